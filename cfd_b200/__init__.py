@@ -888,7 +888,7 @@ class Tuning:
     mixed_sweeps: int = 0  # mixed precision: Jacobi sweeps per level (0: the hierarchy's)
     mixed_weight: float = 0.0  # mixed precision: Jacobi weight (0: the hierarchy's)
     tail_cluster: int = 0  # tail as one cluster of this many CTAs (2..16); 0: cooperative grid
-    vcycle_pair: int = 0  # V-cycle SELL kernels: two rows per thread per pass (1) or one (0)
+    vcycle_pair: int = 0  # V-cycle SELL kernels: next row loaded ahead (1) or one row at a time (0)
     krylov_stage: int = 0  # level-0 Krylov SpMV staged through shared memory in 2..4 buffers; 0: off
 
     def _c(self):

@@ -8,11 +8,11 @@ The knobs are those of `Tuning` (include/cfdb.h, cfdb_tuning):
 * lanes_div    - lanes per CSR row = average row length / lanes_div,
 * fuse_first   - first two Jacobi sweeps of the pre-smoothing fused into one kernel,
 * sell_rows    - rows per CTA of SELL operators (one row per thread per pass),
-* krylov_pair  - level-0 Krylov SpMV kernels take two rows per thread per pass, or one,
+* krylov_pair  - level-0 Krylov SpMV kernels load the next row ahead, or take one at a time,
 * krylov_stage - the level-0 Krylov SpMV streams the operator through shared memory by bulk
                  copies in this many buffers (0: the threads load it, as krylov_pair says),
 * tail_rows    - coarse levels of at most this many rows run in one persistent kernel,
-* vcycle_pair  - V-cycle kernels of SELL operators take two rows per thread per pass, or one,
+* vcycle_pair  - V-cycle kernels of SELL operators load the next row ahead, or take one at a time,
 * tail_cluster - that kernel as one thread-block cluster of this many CTAs (0: a cooperative
                  grid), searched jointly with tail_rows (the candidates keep the grid form),
 * mixed_sweeps, mixed_weight - the smoother schedule of the mixed-precision V-cycle (Jacobi

@@ -111,8 +111,9 @@ SolveResult Engine::solve_bicgstab(const SolveRequest& rq) {
     cudaStream_t st = stream_;
     const int g = bcg_grid(n);
     auto spmv = [&](const double* in, double* out) {
-        k_vc_spmv<double, kVisitSell2><<<d.n_tiles, kBlock, 0, st>>>(d.a.s64, d.tiles, nullptr, in, out, nullptr,
-                                                                     nullptr, 0);
+        auto run = [&](auto kernel) { kernel<<<d.n_tiles, kBlock, 0, st>>>(d.a.s64, d.tiles, nullptr, in, out, nullptr, nullptr, 0); };
+        if (krylov_visit_of(row_width(d.a), true) == kVisitStream5) run(k_vc_spmv<double, kVisitStream5>);
+        else run(k_vc_spmv<double, kVisitStream7>);
         ++launches_;
     };
     std::vector<double> hp(2 * kBcgBlocks);

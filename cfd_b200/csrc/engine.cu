@@ -1049,10 +1049,26 @@ template <> Sell<float> vs_sel<float>(const Sell<double>&, const Sell<float>& b)
 
 // Calls fn with the visiting strategy v as a compile-time constant.
 template <class Fn> void with_visit(int v, Fn&& fn) {
-    if (v == kVisitSell2) fn(std::integral_constant<int, kVisitSell2>{});
-    else if (v == kVisitSell1) fn(std::integral_constant<int, kVisitSell1>{});
-    else if (v == kVisitWarp) fn(std::integral_constant<int, kVisitWarp>{});
-    else fn(std::integral_constant<int, kVisitBlock>{});
+    switch (v) {
+    case kVisitSell4: fn(std::integral_constant<int, kVisitSell4>{}); break;
+    case kVisitSell5: fn(std::integral_constant<int, kVisitSell5>{}); break;
+    case kVisitSell7: fn(std::integral_constant<int, kVisitSell7>{}); break;
+    case kVisitSellLong: fn(std::integral_constant<int, kVisitSellLong>{}); break;
+    case kVisitStream5: fn(std::integral_constant<int, kVisitStream5>{}); break;
+    case kVisitStream7: fn(std::integral_constant<int, kVisitStream7>{}); break;
+    case kVisitWarp: fn(std::integral_constant<int, kVisitWarp>{}); break;
+    default: fn(std::integral_constant<int, kVisitBlock>{}); break;
+    }
+}
+
+// The strategies of krylov_visit_of.
+template <class Fn> void with_krylov_visit(int v, Fn&& fn) {
+    switch (v) {
+    case kVisitSell5: fn(std::integral_constant<int, kVisitSell5>{}); break;
+    case kVisitSell7: fn(std::integral_constant<int, kVisitSell7>{}); break;
+    case kVisitStream5: fn(std::integral_constant<int, kVisitStream5>{}); break;
+    default: fn(std::integral_constant<int, kVisitStream7>{}); break;
+    }
 }
 } // namespace
 
@@ -1400,7 +1416,7 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
             T* o = c == x ? y : x;
             const bool last = k + 1 == sweeps_;
             if (l == 0 && last && fused_final) {
-                with_visit(krylov_visit(), [&](auto V) {
+                with_krylov_visit(krylov_visit(), [&](auto V) {
                     launch_k(tuning_.pdl != 0, k_vc_jacobi_final<T, decltype(V)::value>, d.n_tiles_nc, kBlock, 0, s, 
                         A(0), d.tiles, st_, WD(0), r_, c, o, q_, red_, Control{n_active_, error_, tuning_.wait_polls}, flexible);
                 });
@@ -1430,7 +1446,7 @@ void Engine::enqueue_init(Mode mode) {
     const double a0 = static_cast<double>(d.a.nnz) * 12.0 + 4.0 * (n + 1.0) + 16.0 * n;
     const X1Out x1o = x1_out(mode);
     const double x1b = (mode == Mode::AmgMixed ? 8.0 : 16.0) * x1o.n;
-    with_visit(krylov_visit(), [&](auto V) {
+    with_krylov_visit(krylov_visit(), [&](auto V) {
         launch_k(tuning_.pdl != 0, k_cg_init<decltype(V)::value>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, st_, b_, x_, r_, red_, ctl, x1o);
     });
     mark("cg_init", 0, a0 + 16.0 * n + x1b);
@@ -1509,7 +1525,7 @@ void Engine::enqueue_iteration(Mode mode) {
         else if (tuning_.krylov_stage == 3) staged(k_cg_spmv_pq_staged<3>);
         else staged(k_cg_spmv_pq_staged<4>);
     } else {
-        with_visit(krylov_visit(), [&](auto V) {
+        with_krylov_visit(krylov_visit(), [&](auto V) {
             launch_k(tuning_.pdl != 0, k_cg_spmv_pq<decltype(V)::value>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, st_, p_, q_, red_, ctl);
         });
     }
@@ -1527,7 +1543,7 @@ void Engine::enqueue_iteration(Mode mode) {
     }
     mark("cg_xr", 0, 48.0 * n + x1b);
     if (mode == Mode::AmgMixed) {
-        with_visit(krylov_visit(), [&](auto V) {
+        with_krylov_visit(krylov_visit(), [&](auto V) {
             launch_k(tuning_.pdl != 0, k_cg_true_check<decltype(V)::value>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, st_, b_, x_, r_,
                                                                                red_, ctl, x1o);
         });
@@ -1718,7 +1734,7 @@ std::vector<SolveResult> Engine::solve(Mode mode, const std::vector<SolveRequest
     }
     // true residual for reporting
     const DevLevel& d = lv_[0];
-    with_visit(krylov_visit(), [&](auto V) {
+    with_krylov_visit(krylov_visit(), [&](auto V) {
         launch_k(tuning_.pdl != 0, k_true_residual<decltype(V)::value>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, st_, b_, x_, red_);
     });
     ++launches_;
@@ -1805,30 +1821,6 @@ double Engine::time_sweep(int level, int reps, double* bytes) {
     CFDB_CUDA(cudaEventRecord(b, stream_));
     CFDB_CUDA(cudaEventSynchronize(b));
     CFDB_CUDA(cudaGetLastError());
-    float ms = 0.f;
-    CFDB_CUDA(cudaEventElapsedTime(&ms, a, b));
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    return ms / reps;
-}
-
-double Engine::time_level0_sweep(bool fp32, int reps) {
-    const DevLevel& d = lv_[0];
-    cudaEvent_t a, b;
-    CFDB_CUDA(cudaEventCreate(&a));
-    CFDB_CUDA(cudaEventCreate(&b));
-    CFDB_CUDA(cudaEventRecord(a, stream_));
-    for (int i = 0; i < reps; ++i) {
-        if (fp32) {
-            launch_k(tuning_.pdl != 0, k_vc_jacobi<float, double, kVisitSell2>, d.n_tiles, kBlock, 0, stream_, d.a.s32, d.tiles, nullptr, d.wd32, r_,
-                                                                         d.x32, d.y32);
-        } else {
-            launch_k(tuning_.pdl != 0, k_vc_jacobi<double, double, kVisitSell2>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, nullptr, d.wd64, r_,
-                                                                          d.x64, d.y64);
-        }
-    }
-    CFDB_CUDA(cudaEventRecord(b, stream_));
-    CFDB_CUDA(cudaEventSynchronize(b));
     float ms = 0.f;
     CFDB_CUDA(cudaEventElapsedTime(&ms, a, b));
     cudaEventDestroy(a);

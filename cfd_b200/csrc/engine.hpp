@@ -43,7 +43,8 @@ struct Tuning {
                                 // and at least enough lanes to give ~150K threads per operator
     int fuse_first = 0;         // first two smoothing sweeps in one kernel (x1 recomputed)
     int sell_rows = kSellRows;  // rows per CTA of SELL operators (multiple of kSellRows)
-    int krylov_pair = 1;        // level-0 Krylov SpMV kernels: two rows per thread per pass
+    int krylov_pair = 1;        // level-0 Krylov SpMV kernels: the next row's operands loaded while
+                                // the current row is summed (0: one row at a time)
     int col16 = 0;              // FP32 operators store 16-bit column offsets where they fit
     int tail_rows = 0;          // coarse levels of at most this many rows (and everything below
                                 // them) run as one persistent tail kernel; 0 disables it
@@ -53,8 +54,8 @@ struct Tuning {
     double mixed_weight = 0.0;  // mixed precision: Jacobi weight (0: the hierarchy's)
     int tail_cluster = 0;       // the tail as one thread-block cluster of this many CTAs (2..16)
                                 // separated by the cluster barrier; 0: a cooperative grid
-    int vcycle_pair = 0;        // V-cycle kernels of SELL operators take two rows per thread per
-                                // pass (as the level-0 Krylov kernels with krylov_pair), or one
+    int vcycle_pair = 0;        // V-cycle kernels of SELL operators load the next row's operands
+                                // ahead too (as krylov_pair), or take one row at a time
     int krylov_stage = 0;       // level-0 Krylov SpMV with the operator staged through shared
                                 // memory in this many buffers (2..4); 0: krylov_pair's kernels
 };
@@ -127,8 +128,6 @@ public:
     void set_residual(int s, const double* r, bool device_ptr);
     void get_precond(int s, double* z, bool device_ptr, Mode mode);
 
-    // Kernel timing probe: average device time (ms) of the level-0 FP64/FP32 smoother sweep.
-    double time_level0_sweep(bool fp32, int reps);
     // Average device time (ms) of `reps` back-to-back Jacobi sweeps of level l in the plan's
     // precision and launch shape (level 0 reads the Krylov residual); *bytes = algorithmic bytes
     // of one sweep (operator, weights, right-hand side, iterate in and out).
@@ -198,12 +197,18 @@ private:
     void prepare_stage();
     template <class T> void prepare_tail();
     template <class T> void launch_tail(cudaStream_t s);
-    // rows per thread per pass of the level-0 Krylov SpMV kernels (two, or one)
-    int krylov_visit() const { return tuning_.krylov_pair ? kVisitSell2 : kVisitSell1; }
+    // row-visiting strategy of the level-0 Krylov kernels
+    int krylov_visit() const { return krylov_visit_of(row_width(lv_[0].a), tuning_.krylov_pair != 0); }
     // row-visiting strategy of a V-cycle operator's kernels
     int vcycle_visit(const DevSell64_32& m) const {
-        const int v = visit_of(m.s64.val != nullptr ? m.s64.fmt : m.s32.fmt);
-        return v == kVisitSell1 && tuning_.vcycle_pair ? kVisitSell2 : v;
+        const bool fp64 = m.s64.val != nullptr;
+        const int fmt = fp64 ? m.s64.fmt : m.s32.fmt;
+        if (fmt == kFmtSell && tuning_.vcycle_pair) return krylov_visit_of(row_width(m), true);
+        return visit_of(fmt, row_width(m), m.n_tiles, fp64 && !need32_);
+    }
+    // stored entries per row of a SELL operator
+    static double row_width(const DevSell64_32& m) {
+        return m.n_slices > 0 ? static_cast<double>(m.slots) / (32.0 * m.n_slices) : 0.0;
     }
     // where the residual producers of `mode` write the level-0 first sweep (n = 0: nowhere)
     X1Out x1_out(Mode mode) const;

@@ -28,13 +28,20 @@ constexpr int kBlock = 256;
 // a SELL operator's rows may be reordered by length.
 constexpr int kSellRows = kBlock;
 
-// Programmatic dependent launch (sm_90+): let the next kernel of the stream be scheduled once
-// every CTA of this one has started, then wait until the previous kernel has completed and its
-// writes are visible. Both are no-ops for a kernel launched without the attribute. Every kernel
-// below except the persistent tail calls it first, before touching global memory.
+// Programmatic dependent launch (sm_90+): pdl_launch lets the next kernel of the stream be
+// scheduled once every CTA of this one has started; pdl_wait waits until the previous kernel has
+// completed and its writes are visible. Both are no-ops for a kernel launched without the
+// attribute. Every thread of every kernel below except the persistent tail calls pdl_wait
+// before it leaves or touches anything that another kernel of a solve writes. Between the two
+// calls a kernel reads only what no kernel of a captured graph writes (an operator's offsets,
+// columns and values, its row order and its launch tiles), so that these loads run while the
+// previous kernel finishes. k_fill_level0, which writes level 0's values, is always separated
+// from the kernels that read them by a full stream dependency (a copy or a graph launch).
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_entry() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_launch();
+    pdl_wait();
 }
 
 // Storage of one sparse operator of a level, selected by `fmt`:
@@ -203,118 +210,76 @@ template <class T> __device__ __forceinline__ T madd(T s, T a, T b) {
     else return fmaf(a, b, s);
 }
 
-// Predicated batch of four SELL entries starting at k (column -1 beyond the row end e); C16:
-// compressed columns (the caller has checked m.c16).
-template <bool C16, class T>
-__device__ __forceinline__ void sell_load4(const Sell<T>& m, int k, int e, int base, T (&v)[4], int (&c)[4]) {
+// Predicated batch of B SELL entries starting at slot k (column -1 beyond the slice end e).
+template <int B, class T>
+__device__ __forceinline__ void sell_load(const Sell<T>& m, int k, int e, int base, T (&v)[B], int (&c)[B]) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const bool ok = k + 32 * u < e;
-        v[u] = ok ? __ldg(&m.val[k + 32 * u]) : T(0);
-        if constexpr (C16) c[u] = ok ? base + static_cast<int>(__ldg(&m.c16[k + 32 * u])) : -1;
-        else c[u] = ok ? __ldg(&m.col[k + 32 * u]) : -1;
-    }
-}
-
-template <class T, class XA>
-__device__ __forceinline__ void sell_acc4(T& s, const T (&v)[4], const int (&c)[4], XA xa) {
-    T xv[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) xv[u] = c[u] >= 0 ? xa(c[u]) : T(0);
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-        if (c[u] >= 0) s = madd<T>(s, v[u], xv[u]);
-}
-
-// Row sum of a SELL row: sum_k val[k] * xa(col[k]) in CSR order. Entries are taken in batches
-// of four, software-pipelined: the column / value loads of the next batch are issued before the
-// gathers of the current one, so a thread keeps two batches of the row in flight. Every row of
-// a slice has the slice's width, so the batch predicates are warp-uniform.
-template <bool C16, class T, class XA>
-__device__ __forceinline__ T sell_row_sum_c(const Sell<T>& m, int row, XA xa) {
-    const int slice = row >> 5;
-    const int lane = row & 31;
-    int k = __ldg(&m.slice[slice]) + lane;
-    const int end = __ldg(&m.slice[slice + 1]);
-    const int base = C16 ? __ldg(&m.cbase[slice]) : 0;
-    T s = T(0);
-    if (k >= end) return s;
-    T v[4];
-    int c[4];
-    sell_load4<C16>(m, k, end, base, v, c);
-    for (;;) {
-        k += 128;
-        T vn[4];
-        int cn[4];
-        sell_load4<C16>(m, k, end, base, vn, cn);
-        sell_acc4(s, v, c, xa);
-        if (k >= end) break;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            v[u] = vn[u];
-            c[u] = cn[u];
-        }
-    }
-    return s;
-}
-
-template <class T, class XA>
-__device__ __forceinline__ T sell_row_sum(const Sell<T>& m, int row, XA xa) {
-    if constexpr (sizeof(T) == 4) {
-        if (m.c16 != nullptr) return sell_row_sum_c<true>(m, row, xa);
-    }
-    return sell_row_sum_c<false>(m, row, xa);
-}
-
-// Two SELL rows of one thread, both software-pipelined as in sell_row_sum (up to four batches
-// in flight per thread); each row is still accumulated in its own CSR order.
-template <bool C16, class T, class XA>
-__device__ __forceinline__ void sell_row_sum2_c(const Sell<T>& m, int ra, int rb, XA xa, T& sa, T& sb) {
-    int ka = __ldg(&m.slice[ra >> 5]) + (ra & 31);
-    const int ea = __ldg(&m.slice[(ra >> 5) + 1]);
-    int kb = __ldg(&m.slice[rb >> 5]) + (rb & 31);
-    const int eb = __ldg(&m.slice[(rb >> 5) + 1]);
-    const int ba = C16 ? __ldg(&m.cbase[ra >> 5]) : 0, bb = C16 ? __ldg(&m.cbase[rb >> 5]) : 0;
-    sa = T(0);
-    sb = T(0);
-    T va[4], vb[4];
-    int ca[4], cb[4];
-    sell_load4<C16>(m, ka, ea, ba, va, ca);
-    sell_load4<C16>(m, kb, eb, bb, vb, cb);
-    for (;;) {
-        ka += 128;
-        kb += 128;
-        T van[4], vbn[4];
-        int can[4], cbn[4];
-        sell_load4<C16>(m, ka, ea, ba, van, can);
-        sell_load4<C16>(m, kb, eb, bb, vbn, cbn);
-        sell_acc4(sa, va, ca, xa);
-        sell_acc4(sb, vb, cb, xa);
-        if (ka >= ea && kb >= eb) break;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            va[u] = van[u];
-            ca[u] = can[u];
-            vb[u] = vbn[u];
-            cb[u] = cbn[u];
-        }
-    }
-}
-
-template <class T, class XA>
-__device__ __forceinline__ void sell_row_sum2(const Sell<T>& m, int ra, int rb, XA xa, T& sa, T& sb) {
+    for (int u = 0; u < B; ++u) v[u] = k + 32 * u < e ? __ldg(&m.val[k + 32 * u]) : T(0);
     if constexpr (sizeof(T) == 4) {
         if (m.c16 != nullptr) {
-            sell_row_sum2_c<true>(m, ra, rb, xa, sa, sb);
+#pragma unroll
+            for (int u = 0; u < B; ++u)
+                c[u] = k + 32 * u < e ? base + static_cast<int>(__ldg(&m.c16[k + 32 * u])) : -1;
             return;
         }
     }
-    sell_row_sum2_c<false>(m, ra, rb, xa, sa, sb);
+#pragma unroll
+    for (int u = 0; u < B; ++u) c[u] = k + 32 * u < e ? __ldg(&m.col[k + 32 * u]) : -1;
 }
 
-template <class T, class X>
-__device__ __forceinline__ T sell_row(const Sell<T>& m, int row, const X* __restrict__ x) {
-    return sell_row_sum(m, row, [x](int j) { return static_cast<T>(x[j]); });
+// s += the batch's products, in order; its gathers are in flight together.
+template <int B, class T, class XA>
+__device__ __forceinline__ void sell_acc(T& s, const T (&v)[B], const int (&c)[B], XA xa) {
+    T xv[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) xv[u] = c[u] >= 0 ? xa(c[u]) : T(0);
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+        if (c[u] >= 0) s = madd<T>(s, v[u], xv[u]);
+}
+
+// Where a thread's SELL row starts: first slot, slice end, column base and row number.
+struct SellRow {
+    int k = 0, e = 0, base = 0, row = 0;
+};
+
+template <class T> __device__ __forceinline__ SellRow sell_row_at(const Sell<T>& m, int pos) {
+    SellRow r;
+    const int slice = pos >> 5;
+    r.k = __ldg(&m.slice[slice]) + (pos & 31);
+    r.e = __ldg(&m.slice[slice + 1]);
+    if constexpr (sizeof(T) == 4) r.base = m.c16 != nullptr ? __ldg(&m.cbase[slice]) : 0;
+    r.row = m.perm != nullptr ? __ldg(&m.perm[pos]) : pos;
+    return r;
+}
+
+// Row sum sum_k val[k] * xa(col[k]) in CSR order, the row's first batch (v, c) already loaded.
+// AHEAD: the next batch's columns and values are loaded before the current batch's gathers.
+template <bool AHEAD, int B, class T, class XA>
+__device__ __forceinline__ T sell_sum(const Sell<T>& m, SellRow r, T (&v)[B], int (&c)[B], XA xa) {
+    T s = T(0);
+    if constexpr (AHEAD) {
+        for (;;) {
+            r.k += 32 * B;
+            T vn[B];
+            int cn[B];
+            sell_load<B>(m, r.k, r.e, r.base, vn, cn);
+            sell_acc<B>(s, v, c, xa);
+            if (r.k >= r.e) break;
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                v[u] = vn[u];
+                c[u] = cn[u];
+            }
+        }
+    } else {
+        sell_acc<B>(s, v, c, xa);
+        for (r.k += 32 * B; r.k < r.e; r.k += 32 * B) {
+            sell_load<B>(m, r.k, r.e, r.base, v, c);
+            sell_acc<B>(s, v, c, xa);
+        }
+    }
+    return s;
 }
 
 // Four consecutive values from a 16-byte aligned address.
@@ -357,50 +322,70 @@ __device__ __forceinline__ void ld4col(const Sell<T>& m, int k, int base, int (&
 // columns and values): lane `sub` takes quads sub, sub + G, ... of the row's aligned span, two
 // quads per pass, and masks the entries outside [row begin, row end). CSR arrays carry four
 // entries of slack so the last quad never reads past them.
+template <class T> struct CsrQuads {
+    int b = 0, e = 0, base = 0; // the row's entries and column base
+    int k = 0;                  // first entry of the lane's current pass
+    int c[8];
+    T v[8];
+};
+
+// Columns and values of the lane's pass at q.k (second quad at q.k + 4 G); nothing when the pass
+// starts past the row's end.
+template <class T> __device__ __forceinline__ void csr_load(const Sell<T>& m, int G, CsrQuads<T>& q) {
+    const int k2 = q.k + 4 * G;
+    if (q.k < q.e) {
+        T t[4];
+        ld4col(m, q.k, q.base, q.c, 0);
+        ld4(m.val + q.k, t);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q.v[u] = t[u];
+    }
+    if (k2 < q.e) {
+        T t[4];
+        ld4col(m, k2, q.base, q.c, 4);
+        ld4(m.val + k2, t);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q.v[4 + u] = t[u];
+    }
+}
+
+// The lane's first pass over a row.
+template <class T> __device__ __forceinline__ void csr_begin(const Sell<T>& m, int row, int sub, int G, CsrQuads<T>& q) {
+    q.b = __ldg(&m.slice[row]);
+    q.e = __ldg(&m.slice[row + 1]);
+    q.base = sizeof(T) == 4 && m.c16 != nullptr ? __ldg(&m.cbase[row]) : 0;
+    q.k = (q.b & ~3) + 4 * sub;
+    csr_load(m, G, q);
+}
+
 template <class T, class XA>
-__device__ __forceinline__ T csr_lane_sum(const Sell<T>& m, int row, int sub, int G, XA xa) {
-    const int b = __ldg(&m.slice[row]);
-    const int e = __ldg(&m.slice[row + 1]);
-    const int base = sizeof(T) == 4 && m.c16 != nullptr ? __ldg(&m.cbase[row]) : 0;
+__device__ __forceinline__ T csr_lane_sum(const Sell<T>& m, int G, CsrQuads<T>& q, XA xa) {
     T s = T(0);
-    for (int k = (b & ~3) + 4 * sub; k < e; k += 8 * G) {
-        const int k2 = k + 4 * G;
-        const bool two = k2 < e;
-        int c[8];
-        T v[8], xv[8];
-        {
-            ld4col(m, k, base, c, 0);
-            T t[4];
-            ld4(m.val + k, t);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = t[u];
-        }
-        if (two) {
-            ld4col(m, k2, base, c, 4);
-            T t[4];
-            ld4(m.val + k2, t);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) v[4 + u] = t[u];
-        }
+    for (; q.k < q.e;) {
+        const int k2 = q.k + 4 * G;
+        const bool two = k2 < q.e;
+        T xv[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const int kk = (u < 4 ? k : k2) + (u & 3);
-            const bool ok = (u < 4 || two) && kk >= b && kk < e;
-            xv[u] = ok ? xa(c[u]) : T(0);
-            if (!ok) v[u] = T(0);
+            const int kk = (u < 4 ? q.k : k2) + (u & 3);
+            const bool ok = (u < 4 || two) && kk >= q.b && kk < q.e;
+            xv[u] = ok ? xa(q.c[u]) : T(0);
+            if (!ok) q.v[u] = T(0);
         }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) s = madd<T>(s, v[u], xv[u]);
+        for (int u = 0; u < 8; ++u) s = madd<T>(s, q.v[u], xv[u]);
+        q.k += 8 * G;
+        csr_load(m, G, q);
     }
     return s;
 }
 
-// CSR row sum by a group of G lanes (G a power of two dividing 32); partial sums are combined
-// with a fixed butterfly over the group. Every lane of the group returns the same total. All
+// CSR row sum by a group of G lanes (G a power of two dividing 32), each with its first pass over
+// the row loaded (csr_begin); partial sums are combined with a fixed butterfly over the group. Every lane of the group returns the same total. All
 // lanes of the warp must call it (the shuffles use the full mask).
 template <class T, class XA>
-__device__ __forceinline__ T csr_group_sum(const Sell<T>& m, int row, bool valid, int sub, int G, XA xa) {
-    T s = valid ? csr_lane_sum(m, row, sub, G, xa) : T(0);
+__device__ __forceinline__ T csr_group_sum(const Sell<T>& m, CsrQuads<T>& q, bool valid, int G, XA xa) {
+    T s = valid ? csr_lane_sum(m, G, q, xa) : T(0);
     for (int o = G >> 1; o > 0; o >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, o);
     return s;
 }
@@ -409,9 +394,9 @@ __device__ __forceinline__ T csr_group_sum(const Sell<T>& m, int row, bool valid
 // butterfly within each warp, then the row's warps are added in warp order. Returns the
 // total in the row's first lane. Every thread of the block must call it (__syncthreads).
 template <class T, class XA>
-__device__ __forceinline__ T csr_block_sum(const Sell<T>& m, int row, bool valid, int sub, int G, XA xa) {
+__device__ __forceinline__ T csr_block_sum(const Sell<T>& m, CsrQuads<T>& q, bool valid, int sub, int G, XA xa) {
     __shared__ T red[kBlock / 32];
-    T s = valid ? csr_lane_sum(m, row, sub, G, xa) : T(0);
+    T s = valid ? csr_lane_sum(m, G, q, xa) : T(0);
     for (int o = 16; o > 0; o >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, o);
     const int w = static_cast<int>(threadIdx.x) >> 5;
     if ((threadIdx.x & 31) == 0) red[w] = s;
@@ -425,8 +410,6 @@ __device__ __forceinline__ T csr_block_sum(const Sell<T>& m, int row, bool valid
     return t;
 }
 
-struct TileCtx;
-
 // Rows of a fine tile (CSR operators with G <= 32): one group of G = fmt lanes per row,
 // blockDim = 8 * G. Wider groups take 256 / G rows per tile with blockDim 256.
 constexpr int kFineRows = 8;
@@ -434,98 +417,152 @@ constexpr int kFineRows = 8;
 
 // Row-visiting strategies of the tiled kernels, fixed at compile time so that each kernel
 // instance holds the registers of one strategy only:
-//  kVisitSell2  SELL, two rows per thread per pass (big tiles of the Krylov kernels, and the
-//               V-cycle kernels with Tuning.vcycle_pair), rows optionally reordered;
-//  kVisitSell1  SELL, one row per thread per pass, rows optionally reordered (V-cycle kernels);
-//  kVisitWarp   CSR, G <= 32 lanes per row (8 rows per tile);
-//  kVisitBlock  CSR, G = 64..256 lanes per row (256 / G rows per tile).
-enum : int { kVisitSell2 = 0, kVisitSell1 = 1, kVisitWarp = 2, kVisitBlock = 3 };
+//  kVisitSell4/5/7  SELL, one row per thread per pass, the row's first 4, 5 or 7 entries taken in
+//                   one batch (their gathers in flight together), the rest in further batches;
+//  kVisitSellLong   the same with batches of 8 and half the CTAs per SM, for operators with long
+//                   rows and too few of them to fill the GPU several times over;
+//  kVisitStream5/7  SELL, batches of 5 or 7, the next row's operands loaded while the current row
+//                   is summed (tiles of many rows per thread: the level-0 Krylov kernels);
+//  kVisitWarp       CSR, G <= 32 lanes per row (8 rows per tile);
+//  kVisitBlock      CSR, G = 64..256 lanes per row (256 / G rows per tile).
+// Every strategy of an operator's format sums each row in the same order.
+enum : int {
+    kVisitSell4 = 0,
+    kVisitSell5,
+    kVisitSell7,
+    kVisitSellLong,
+    kVisitStream5,
+    kVisitStream7,
+    kVisitWarp,
+    kVisitBlock
+};
 
-// Calls f(row, sum_j a_row,j xa(j)) for every row of the tile.
-template <int V, class T, class XA, class F>
-__device__ __forceinline__ void visit_rows_v(const Sell<T>& m, int r0, int r1, XA xa, F f) {
-    if constexpr (V == kVisitSell2) {
-        int row = r0 + threadIdx.x;
-        auto at = [&](int q) { return m.perm != nullptr ? __ldg(&m.perm[q]) : q; };
-        for (; row + kBlock < r1; row += 2 * kBlock) {
-            T s0, s1;
-            sell_row_sum2(m, row, row + kBlock, xa, s0, s1);
-            f(at(row), s0);
-            f(at(row + kBlock), s1);
-        }
-        if (row < r1) f(at(row), sell_row_sum(m, row, xa));
-    } else if constexpr (V == kVisitSell1) {
-        // reordered operators: tiles are aligned windows of positions
-        for (int row = r0 + threadIdx.x; row < r1; row += kBlock)
-            f(m.perm != nullptr ? __ldg(&m.perm[row]) : row, sell_row_sum(m, row, xa));
-    } else {
-        const int G = m.fmt;
-        const int row = r0 + static_cast<int>(threadIdx.x) / G;
-        const int sub = static_cast<int>(threadIdx.x) & (G - 1);
-        const bool valid = row < r1;
-        if constexpr (V == kVisitWarp) {
-            const T s = csr_group_sum(m, row, valid, sub, G, xa);
-            if (valid && sub == 0) f(row, s);
+template <int V> constexpr bool kIsSell = V <= kVisitStream7;
+template <int V> constexpr bool kIsStream = V == kVisitStream5 || V == kVisitStream7;
+template <int V>
+constexpr int kBatch = V == kVisitSell4 ? 4 : V == kVisitSell5 || V == kVisitStream5 ? 5 : V == kVisitSellLong ? 8 : 7;
+
+// One tile's visit: begin() issues the loads of the thread's first row that depend on the
+// operator alone (before pdl_wait); run() calls f(row, sum_j a_row,j xa(j), e) for every row of
+// the tile, with the row's other operands e = pre(row) loaded ahead of its gathers.
+//
+// What bounds these kernels is the chain of dependent loads of a row (slice offsets, columns and
+// values, gathers) against the few rows that a thread has in flight, so a row's entries are taken
+// in as few batches as its width allows and the chain's first part overlaps the previous kernel.
+// Measured against batches of four behind pdl_wait (operands after the sum), back to back, on
+// the tet box of 5.1M cells (5 entries a row): FP32 residual 61.7 -> 52.6 us, FP32 prolongation
+// (3 entries) 52.9 -> 40.6 us; on the graded box of 885K cells (7 entries): FP32 residual
+// 9.4 -> 6.7 us, FP64 14.8 -> 14.0 us, FP32 level-1 residual (42 entries, 146K rows, batches of
+// 8) 11.2 -> 8.3 us, FP64 20.1 -> 13.5 us.
+template <int V, class T> struct Visit {
+    static constexpr bool kSell = kIsSell<V>;
+    static constexpr bool kStream = kIsStream<V>;
+    static constexpr int B = kBatch<V>;
+    // FP32 rows longer than a batch load the next batch ahead of the current gathers; in FP64
+    // the registers for it cost more than it gives (17.5 against 13.5 us on the level above)
+    static constexpr bool kAhead = V == kVisitSellLong && sizeof(T) == 4;
+    SellRow r, rn;
+    T v[kSell ? B : 1];
+    int c[kSell ? B : 1];
+    CsrQuads<T> q;
+
+    __device__ __forceinline__ void begin(const Sell<T>& m, int r0, int r1) {
+        if constexpr (kSell) {
+            const int pos = r0 + static_cast<int>(threadIdx.x);
+            if (pos < r1) r = sell_row_at(m, pos);
+            sell_load<B>(m, r.k, r.e, r.base, v, c);
+            if constexpr (kStream) {
+                if (pos + kBlock < r1) rn = sell_row_at(m, pos + kBlock);
+            }
         } else {
-            const T s = csr_block_sum(m, row, valid, sub, G, xa);
-            if (valid && sub == 0) f(row, s);
+            const int G = m.fmt;
+            const int row = r0 + static_cast<int>(threadIdx.x) / G;
+            if (row < r1) csr_begin(m, row, static_cast<int>(threadIdx.x) & (G - 1), G, q);
         }
     }
-}
 
-// As visit_rows_v, with each row's epilogue operands loaded ahead of its sum: e = pre(row) is
-// issued before the row's column / value loads, so the loads of p[row], b[row], ... overlap the
-// sum instead of following it; then f(row, sum, e). The arithmetic is unchanged. Measured on
-// the jittered tet box (5.1M cells): the level-0 Krylov SpMV 104 -> 91 us and the level-0
-// residual 73 -> 70 us gain from it; the one-row SELL sweeps, prolongations and restrictions
-// (32 registers at full occupancy) lost 3-7 %, so they keep visit_rows_v.
-template <int V, class T, class XA, class P, class F>
-__device__ __forceinline__ void visit_rows_e(const Sell<T>& m, int r0, int r1, XA xa, P pre, F f) {
-    if constexpr (V == kVisitSell2) {
-        int row = r0 + threadIdx.x;
-        auto at = [&](int q) { return m.perm != nullptr ? __ldg(&m.perm[q]) : q; };
-        for (; row + kBlock < r1; row += 2 * kBlock) {
-            const int ra = at(row), rb = at(row + kBlock);
-            const auto e0 = pre(ra);
-            const auto e1 = pre(rb);
-            T s0, s1;
-            sell_row_sum2(m, row, row + kBlock, xa, s0, s1);
-            f(ra, s0, e0);
-            f(rb, s1, e1);
+    template <class XA, class P, class F>
+    __device__ __forceinline__ void run(const Sell<T>& m, int r0, int r1, XA xa, P pre, F f) {
+        if constexpr (kStream) {
+            for (int pos = r0 + static_cast<int>(threadIdx.x); pos < r1; pos += kBlock) {
+                T vn[B];
+                int cn[B];
+                SellRow r2;
+                sell_load<B>(m, rn.k, rn.e, rn.base, vn, cn);
+                if (pos + 2 * kBlock < r1) r2 = sell_row_at(m, pos + 2 * kBlock);
+                const auto e = pre(r.row);
+                f(r.row, sell_sum<false, B>(m, r, v, c, xa), e);
+                r = rn;
+                rn = r2;
+#pragma unroll
+                for (int u = 0; u < B; ++u) {
+                    v[u] = vn[u];
+                    c[u] = cn[u];
+                }
+            }
+        } else if constexpr (kSell) {
+            for (int pos = r0 + static_cast<int>(threadIdx.x); pos < r1;) {
+                const auto e = pre(r.row);
+                f(r.row, sell_sum<kAhead, B>(m, r, v, c, xa), e);
+                pos += kBlock;
+                if (pos < r1) {
+                    r = sell_row_at(m, pos);
+                    sell_load<B>(m, r.k, r.e, r.base, v, c);
+                }
+            }
+        } else {
+            const int G = m.fmt;
+            const int row = r0 + static_cast<int>(threadIdx.x) / G;
+            const int sub = static_cast<int>(threadIdx.x) & (G - 1);
+            const bool valid = row < r1;
+            decltype(pre(0)) e{};
+            if (valid && sub == 0) e = pre(row);
+            T s;
+            if constexpr (V == kVisitWarp) s = csr_group_sum(m, q, valid, G, xa);
+            else s = csr_block_sum(m, q, valid, sub, G, xa);
+            if (valid && sub == 0) f(row, s, e);
         }
-        if (row < r1) {
-            const int ra = at(row);
-            const auto e = pre(ra);
-            f(ra, sell_row_sum(m, row, xa), e);
-        }
-    } else if constexpr (V == kVisitSell1) {
-        for (int row = r0 + threadIdx.x; row < r1; row += kBlock) {
-            const int rr = m.perm != nullptr ? __ldg(&m.perm[row]) : row;
-            const auto e = pre(rr);
-            f(rr, sell_row_sum(m, row, xa), e);
-        }
-    } else {
-        const int G = m.fmt;
-        const int row = r0 + static_cast<int>(threadIdx.x) / G;
-        const int sub = static_cast<int>(threadIdx.x) & (G - 1);
-        const bool valid = row < r1;
-        decltype(pre(0)) e{};
-        if (valid && sub == 0) e = pre(row);
-        T s;
-        if constexpr (V == kVisitWarp) s = csr_group_sum(m, row, valid, sub, G, xa);
-        else s = csr_block_sum(m, row, valid, sub, G, xa);
-        if (valid && sub == 0) f(row, s, e);
     }
+};
+
+struct NoOperands {};
+
+// CTAs per SM the kernels are compiled for. kHeavy: kernels with three operands of their own per
+// row (the Jacobi sweeps) beside the row's batch.
+template <class T, int V, bool kHeavy>
+constexpr int kMinBlocks = sizeof(T) == 4
+                               ? (V == kVisitSell4 || V == kVisitSell5 ? 8
+                                  : V == kVisitSell7                   ? (kHeavy ? 6 : 8)
+                                  : V == kVisitSellLong                ? 4
+                                  : V == kVisitStream5                 ? 4
+                                  : V == kVisitStream7                 ? 3
+                                                                       : 6)
+                               : (V == kVisitSell4     ? (kHeavy ? 6 : 8)
+                                  : V == kVisitSell5   ? 6
+                                  : V == kVisitSell7   ? (kHeavy ? 4 : 6)
+                                  : V == kVisitStream7 ? 3
+                                                       : 4);
+
+// Strategy of an operator's V-cycle kernels. `width`: stored entries per SELL row; `tiles`: its
+// CTAs. The batch is the narrowest that holds a typical row; rows beyond 8 entries take batches
+// of 7 (FP32) or 4 (FP64) while the operator gives every SM more than two rounds of the long form's
+// four CTAs, and the long form below that.
+__host__ __device__ inline int visit_of(int fmt, double width, int tiles, bool fp64) {
+    if (fmt != kFmtSell) return fmt <= 32 ? kVisitWarp : kVisitBlock;
+    if (width <= 4.0) return kVisitSell4;
+    if (width <= 5.25) return kVisitSell5;
+    if (width <= 8.0) return kVisitSell7;
+    if (tiles <= 2 * 4 * 148) return kVisitSellLong;
+    return fp64 ? kVisitSell4 : kVisitSell7;
 }
 
-// CTAs per SM the V-cycle kernels are compiled for: the one-row SELL sweeps fit in 32
-// registers (full occupancy); the lane-group and two-row kernels hold more (FP64 most).
-template <class T, int V>
-constexpr int kMinBlocks = V == kVisitSell1 ? 8 : (sizeof(T) == 8 || V == kVisitSell2 ? 4 : 6);
-
-// Strategy of an operator's V-cycle kernels.
-__host__ __device__ inline int visit_of(int fmt) {
-    return fmt == kFmtSell ? kVisitSell1 : (fmt <= 32 ? kVisitWarp : kVisitBlock);
+// Strategy of the level-0 Krylov kernels (FP64 operands, big tiles): the stream forms, or the
+// one-row forms (ahead = false). On the tet box of 5.1M cells q = A p with its dot takes 67 us
+// streamed (tiles of 1024 to 4352 rows) against 86 us for two rows per thread in batches of four;
+// on the graded box of 885K cells 11.4 against 15.5 us.
+__host__ __device__ inline int krylov_visit_of(double width, bool ahead) {
+    if (width <= 5.25) return ahead ? kVisitStream5 : kVisitSell5;
+    return ahead ? kVisitStream7 : kVisitSell7;
 }
 
 // Tile bookkeeping shared by all tiled kernels.
@@ -533,12 +570,24 @@ struct TileCtx {
     int tile, s, r0, r1;
 };
 
-__device__ __forceinline__ bool tile_begin(const Tiles& t, const SysState* st, TileCtx& c) {
+// This CTA's tile (constant data: may precede pdl_wait).
+__device__ __forceinline__ TileCtx tile_of(const Tiles& t) {
+    TileCtx c;
     c.tile = blockIdx.x;
     c.s = t.sys != nullptr ? __ldg(&t.sys[c.tile]) : 0;  // null: a single system
     c.r0 = __ldg(&t.row[c.tile]);
     c.r1 = __ldg(&t.row[c.tile + 1]);
+    return c;
+}
+
+// Whether the tile's system still iterates (after pdl_wait).
+__device__ __forceinline__ bool tile_active(const SysState* st, const TileCtx& c) {
     return st == nullptr || *((volatile const int*)&st[c.s].active) != 0;
+}
+
+__device__ __forceinline__ bool tile_begin(const Tiles& t, const SysState* st, TileCtx& c) {
+    c = tile_of(t);
+    return tile_active(st, c);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -650,16 +699,25 @@ struct X1Out {
     }
 };
 
+// Operands of a row's Jacobi update besides its sum.
+template <class T, class B> struct JacobiRow {
+    T x, wd;
+    B b;
+};
+
 // First smoothing step from x = 0: x1 = 0 + wd * b (t = A*0 = 0), and when fused2 also the
 // second sweep y = x1 + wd (b - A x1) with x1 of the neighbours recomputed on the fly.
 template <class T, class B, int V>
-static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V>)) k_vc_first(Sell<T> a, Tiles tiles, const SysState* st,
+static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V, true>)) k_vc_first(Sell<T> a, Tiles tiles, const SysState* st,
                                                      const T* __restrict__ wd,
                                                      const B* __restrict__ b, T* __restrict__ y,
                                                      int fused2) {
-    pdl_entry();
-    TileCtx c;
-    if (!tile_begin(tiles, st, c)) return;
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    Visit<V, T> vis;
+    if (fused2) vis.begin(a, c.r0, c.r1);
+    pdl_wait();
+    if (!tile_active(st, c)) return;
     auto x1 = [&](int j) -> T {
         if constexpr (sizeof(T) == 8) return __dadd_rn(0.0, __dmul_rn(wd[j], static_cast<T>(b[j])));
         else return wd[j] * static_cast<T>(b[j]);
@@ -668,68 +726,80 @@ static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V>)) k_vc_first(
         for (int row = c.r0 + threadIdx.x; row < c.r1; row += blockDim.x) y[row] = x1(row);
         return;
     }
-    visit_rows_v<V>(a, c.r0, c.r1, x1, [&](int row, T s) {
-        y[row] = jac_update<T>(x1(row), wd[row], static_cast<T>(b[row]), s);
-    });
+    vis.run(a, c.r0, c.r1, x1, [&](int row) { return JacobiRow<T, B>{x1(row), wd[row], b[row]}; },
+            [&](int row, T s, const JacobiRow<T, B>& o) { y[row] = jac_update<T>(o.x, o.wd, static_cast<T>(o.b), s); });
 }
 
 // y = x + wd (b - A x)
 template <class T, class B, int V>
-static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V>)) k_vc_jacobi(Sell<T> a, Tiles tiles, const SysState* st,
+static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V, true>)) k_vc_jacobi(Sell<T> a, Tiles tiles, const SysState* st,
                                                       const T* __restrict__ wd,
                                                       const B* __restrict__ b,
                                                       const T* __restrict__ x, T* __restrict__ y) {
-    pdl_entry();
-    TileCtx c;
-    if (!tile_begin(tiles, st, c)) return;
-    visit_rows_v<V>(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row, T s) {
-        y[row] = jac_update<T>(x[row], wd[row], static_cast<T>(b[row]), s);
-    });
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    Visit<V, T> vis;
+    vis.begin(a, c.r0, c.r1);
+    pdl_wait();
+    if (!tile_active(st, c)) return;
+    vis.run(a, c.r0, c.r1, [x](int j) { return x[j]; },
+            [&](int row) { return JacobiRow<T, B>{x[row], wd[row], b[row]}; },
+            [&](int row, T s, const JacobiRow<T, B>& o) { y[row] = jac_update<T>(o.x, o.wd, static_cast<T>(o.b), s); });
 }
 
 // t = b - A x
 template <class T, class B, int V>
-static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V>)) k_vc_residual(Sell<T> a, Tiles tiles, const SysState* st,
+static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V, false>)) k_vc_residual(Sell<T> a, Tiles tiles, const SysState* st,
                                                         const B* __restrict__ b,
                                                         const T* __restrict__ x,
                                                         T* __restrict__ t) {
-    pdl_entry();
-    TileCtx c;
-    if (!tile_begin(tiles, st, c)) return;
-    visit_rows_e<V>(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row) { return b[row]; },
-                    [&](int row, T s, B bi) {
-                        if constexpr (sizeof(T) == 8) t[row] = __dsub_rn(static_cast<T>(bi), s);
-                        else t[row] = static_cast<T>(bi) - s;
-                    });
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    Visit<V, T> vis;
+    vis.begin(a, c.r0, c.r1);
+    pdl_wait();
+    if (!tile_active(st, c)) return;
+    vis.run(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row) { return b[row]; }, [&](int row, T s, B bi) {
+        if constexpr (sizeof(T) == 8) t[row] = __dsub_rn(static_cast<T>(bi), s);
+        else t[row] = static_cast<T>(bi) - s;
+    });
 }
 
 // y = M x (restriction into the next level's right-hand side)
 template <class T, int V>
-static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V>)) k_vc_spmv(Sell<T> m, Tiles tiles, const SysState* st,
+static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V, false>)) k_vc_spmv(Sell<T> m, Tiles tiles, const SysState* st,
                                                     const T* __restrict__ x, T* __restrict__ y,
                                                     const T* __restrict__ wd1, T* __restrict__ x1,
                                                     int n1) {
-    pdl_entry();
-    TileCtx c;
-    if (!tile_begin(tiles, st, c)) return;
-    visit_rows_v<V>(m, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row, T s) {
-        y[row] = s;
-        // restriction: also the first pre-smoothing sweep of the coarser level
-        if (x1 != nullptr && row < n1) x1[row] = first_sweep<T>(wd1[row], s);
-    });
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    Visit<V, T> vis;
+    vis.begin(m, c.r0, c.r1);
+    pdl_wait();
+    if (!tile_active(st, c)) return;
+    vis.run(m, c.r0, c.r1, [x](int j) { return x[j]; },
+            [&](int row) { return x1 != nullptr && row < n1 ? wd1[row] : T(0); },
+            [&](int row, T s, T w) {
+                y[row] = s;
+                // restriction: also the first pre-smoothing sweep of the coarser level
+                if (x1 != nullptr && row < n1) x1[row] = first_sweep<T>(w, s);
+            });
 }
 
 // x += P xc
 template <class T, int V>
-static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V>)) k_vc_prolong(Sell<T> p, Tiles tiles, const SysState* st,
+static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V, false>)) k_vc_prolong(Sell<T> p, Tiles tiles, const SysState* st,
                                                        const T* __restrict__ xc,
                                                        T* __restrict__ x) {
-    pdl_entry();
-    TileCtx c;
-    if (!tile_begin(tiles, st, c)) return;
-    visit_rows_v<V>(p, c.r0, c.r1, [xc](int j) { return xc[j]; }, [&](int row, T s) {
-        if constexpr (sizeof(T) == 8) x[row] = __dadd_rn(x[row], s);
-        else x[row] = x[row] + s;
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    Visit<V, T> vis;
+    vis.begin(p, c.r0, c.r1);
+    pdl_wait();
+    if (!tile_active(st, c)) return;
+    vis.run(p, c.r0, c.r1, [xc](int j) { return xc[j]; }, [&](int row) { return x[row]; }, [&](int row, T s, T xi) {
+        if constexpr (sizeof(T) == 8) x[row] = __dadd_rn(xi, s);
+        else x[row] = xi + s;
     });
 }
 
@@ -857,9 +927,9 @@ static __global__ void __launch_bounds__(kBlock) k_vc_coarse(CoarseBlocks cb, co
 // Thread 0 keeps S - 1 chunks in flight while the block sums the current one from shared
 // memory: a row's gathers then follow a shared-memory load of its columns instead of a DRAM
 // load, and the bytes in flight cost no registers. Each thread takes position c0 + threadIdx.x
-// of every chunk, the order in which kVisitSell1 and kVisitSell2 visit a tile, and sums each
+// of every chunk, the order in which the other SELL strategies visit a tile, and sums each
 // row in CSR order, so rows, sums and the per-thread epilogue order are theirs bit for bit. A
-// chunk with more slots than a stage holds is summed from global memory as kVisitSell1 does.
+// chunk with more slots than a stage holds is summed from global memory.
 
 __device__ __forceinline__ void mbar_init1(uint64_t* bar) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(1) : "memory");
@@ -895,7 +965,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int po
 
 // Sum of one row of a staged chunk: k = the row's first slot and e = its slice's end, both
 // relative to the chunk's first slot. Eight entries per batch, their gathers in flight
-// together; entries in CSR order, padding (column -1) skipped, as sell_row_sum.
+// together; entries in CSR order, padding (column -1) skipped, as sell_sum.
 template <class T, class XA>
 __device__ __forceinline__ T staged_row_sum(const T* sv, const int* sc, int k, int e, XA xa) {
     T s = T(0);
@@ -913,7 +983,7 @@ __device__ __forceinline__ T staged_row_sum(const T* sv, const int* sc, int k, i
     return s;
 }
 
-// As visit_rows_e over the SELL positions [r0, r1) (r0 a multiple of 32), with the operator
+// As Visit::run over the SELL positions [r0, r1) (r0 a multiple of 32), with the operator
 // staged in S buffers of `cap` slots each (dynamic shared memory: S * cap * (sizeof(T) + 4)
 // bytes, cap a multiple of 32). Returns false when a bounded wait expired: ctl.error is set,
 // the CTA's copies in flight have been waited out (bounded too) and the remaining rows are
@@ -988,7 +1058,11 @@ __device__ __forceinline__ bool visit_rows_staged(const Sell<T>& m, int r0, int 
                 sum = staged_row_sum(sval + static_cast<size_t>(s) * cap, scol + static_cast<size_t>(s) * cap,
                                      __ldg(&m.slice[sl]) - first + (pos & 31), __ldg(&m.slice[sl + 1]) - first, xa);
             } else {
-                sum = sell_row_sum(m, pos, xa);
+                T v[4];
+                int c[4];
+                const SellRow r = sell_row_at(m, pos);
+                sell_load<4>(m, r.k, r.e, r.base, v, c);
+                sum = sell_sum<true, 4>(m, r, v, c, xa);
             }
             f(row, sum, e);
         }
@@ -1002,16 +1076,19 @@ __device__ __forceinline__ bool visit_rows_staged(const Sell<T>& m, int r0, int 
 
 // r = b - A x ; |r|_2 ; stop if already converged (iterations = 0)
 template <int V>
-static __global__ void __launch_bounds__(kBlock) k_cg_init(Sell<double> a, Tiles tiles, SysState* st,
+static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>)) k_cg_init(Sell<double> a, Tiles tiles, SysState* st,
                                                     const double* __restrict__ b,
                                                     const double* __restrict__ x,
                                                     double* __restrict__ r, Reduce red,
                                                     Control ctl, X1Out x1o) {
-    pdl_entry();
-    TileCtx c;
-    if (!tile_begin(tiles, st, c)) return;
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    Visit<V, double> vis;
+    vis.begin(a, c.r0, c.r1);
+    pdl_wait();
+    if (!tile_active(st, c)) return;
     double rr = 0.0, unused = 0.0;
-    visit_rows_e<V>(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row) { return b[row]; },
+    vis.run(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row) { return b[row]; },
                     [&](int row, double ax, double bi) {
                         const double ri = __dsub_rn(bi, ax);
                         r[row] = ri;
@@ -1104,15 +1181,18 @@ static __global__ void __launch_bounds__(kBlock) k_cg_spmv_pq_staged(Sell<double
 
 // q = A p ; p.q ; alpha = rz / pq (break if pq == 0)
 template <int V>
-static __global__ void __launch_bounds__(kBlock) k_cg_spmv_pq(Sell<double> a, Tiles tiles, SysState* st,
+static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>)) k_cg_spmv_pq(Sell<double> a, Tiles tiles, SysState* st,
                                                        const double* __restrict__ p,
                                                        double* __restrict__ q, Reduce red,
                                                        Control ctl) {
-    pdl_entry();
-    TileCtx c;
-    if (!tile_begin(tiles, st, c)) return;
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    Visit<V, double> vis;
+    vis.begin(a, c.r0, c.r1);
+    pdl_wait();
+    if (!tile_active(st, c)) return;
     double pq = 0.0;
-    visit_rows_e<V>(a, c.r0, c.r1, [p](int j) { return p[j]; }, [&](int row) { return p[row]; },
+    vis.run(a, c.r0, c.r1, [p](int j) { return p[j]; }, [&](int row) { return p[row]; },
                     [&](int row, double qi, double pi) {
                         q[row] = qi;
                         pq = __dadd_rn(pq, __dmul_rn(pi, qi));
@@ -1185,7 +1265,7 @@ static __global__ void __launch_bounds__(kBlock, (X1 == 0 ? 5 : 4)) k_cg_xr(Tile
 // Mixed precision: for systems whose recursive residual met the target, recompute
 // r = b - A x in FP64; converged if |r| <= tol, else restart the search direction.
 template <int V>
-static __global__ void __launch_bounds__(kBlock) k_cg_true_check(Sell<double> a, Tiles tiles, SysState* st,
+static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>)) k_cg_true_check(Sell<double> a, Tiles tiles, SysState* st,
                                                           const double* __restrict__ b,
                                                           const double* __restrict__ x,
                                                           double* __restrict__ r, Reduce red,
@@ -1195,7 +1275,9 @@ static __global__ void __launch_bounds__(kBlock) k_cg_true_check(Sell<double> a,
     if (!tile_begin(tiles, st, c)) return;
     if (st[c.s].check == 0) return;
     double rr = 0.0, unused = 0.0;
-    visit_rows_e<V>(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row) { return b[row]; },
+    Visit<V, double> vis;
+    vis.begin(a, c.r0, c.r1);
+    vis.run(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row) { return b[row]; },
                     [&](int row, double ax, double bi) {
                         const double ri = __dsub_rn(bi, ax);
                         r[row] = ri;
@@ -1240,7 +1322,7 @@ __device__ __forceinline__ void precond_tail(SysState& s, double rz_new, double 
 
 // Last post-smoothing sweep of level 0 fused with r.z (and z.q): z = x + wd (b - A x).
 template <class T, int V>
-static __global__ void __launch_bounds__(kBlock) k_vc_jacobi_final(Sell<T> a, Tiles tiles, SysState* st,
+static __global__ void __launch_bounds__(kBlock, (kMinBlocks<T, V, true>)) k_vc_jacobi_final(Sell<T> a, Tiles tiles, SysState* st,
                                                             const T* __restrict__ wd,
                                                             const double* __restrict__ r,
                                                             const T* __restrict__ x,
@@ -1248,18 +1330,26 @@ static __global__ void __launch_bounds__(kBlock) k_vc_jacobi_final(Sell<T> a, Ti
                                                             const double* __restrict__ q,
                                                             Reduce red, Control ctl,
                                                             int flexible) {
-    pdl_entry();
-    TileCtx c;
-    if (!tile_begin(tiles, st, c)) return;
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    Visit<V, T> vis;
+    vis.begin(a, c.r0, c.r1);
+    pdl_wait();
+    if (!tile_active(st, c)) return;
     double rz = 0.0, zq = 0.0;
-    visit_rows_v<V>(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row, T s) {
-        const double ri = r[row];
-        const T zi = jac_update<T>(x[row], wd[row], static_cast<T>(ri), s);
-        z[row] = zi;
-        const double zd = static_cast<double>(zi);
-        rz = __dadd_rn(rz, __dmul_rn(ri, zd));
-        if (flexible) zq = __dadd_rn(zq, __dmul_rn(zd, q[row]));
-    });
+    struct Row {
+        T x, wd;
+        double r, q;
+    };
+    vis.run(a, c.r0, c.r1, [x](int j) { return x[j]; },
+            [&](int row) { return Row{x[row], wd[row], r[row], flexible ? q[row] : 0.0}; },
+            [&](int row, T s, const Row& o) {
+                const T zi = jac_update<T>(o.x, o.wd, static_cast<T>(o.r), s);
+                z[row] = zi;
+                const double zd = static_cast<double>(zi);
+                rz = __dadd_rn(rz, __dmul_rn(o.r, zd));
+                if (flexible) zq = __dadd_rn(zq, __dmul_rn(zd, o.q));
+            });
     if (reduce_system(rz, zq, c.tile, c.s, red) && threadIdx.x == 0) {
         precond_tail(st[c.s], rz, zq, flexible, ctl);
     }
@@ -1316,18 +1406,21 @@ static __global__ void __launch_bounds__(kBlock) k_cg_rz(Tiles tiles, SysState* 
 
 // |b - A x|_2 per system into st.true_res (reporting only; all systems).
 template <int V>
-static __global__ void __launch_bounds__(kBlock) k_true_residual(Sell<double> a, Tiles tiles, SysState* st,
+static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>)) k_true_residual(Sell<double> a, Tiles tiles, SysState* st,
                                                           const double* __restrict__ b,
                                                           const double* __restrict__ x,
                                                           Reduce red) {
-    pdl_entry();
-    TileCtx c;
-    tile_begin(tiles, nullptr, c);
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    Visit<V, double> vis;
+    vis.begin(a, c.r0, c.r1);
+    pdl_wait();
     double rr = 0.0, unused = 0.0;
-    visit_rows_v<V>(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row, double ax) {
-        const double ri = __dsub_rn(b[row], ax);
-        rr = __dadd_rn(rr, __dmul_rn(ri, ri));
-    });
+    vis.run(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row) { return b[row]; },
+            [&](int, double ax, double bi) {
+                const double ri = __dsub_rn(bi, ax);
+                rr = __dadd_rn(rr, __dmul_rn(ri, ri));
+            });
     if (reduce_system(rr, unused, c.tile, c.s, red) && threadIdx.x == 0) {
         st[c.s].true_res = sqrt(rr);
     }
@@ -1543,9 +1636,11 @@ __device__ __forceinline__ void tail_rows(const Sell<T>& m, int n, XA xa, F f) {
     for (int base = blockIdx.x * rpb; base < n; base += gridDim.x * rpb) {
         const int row = base + static_cast<int>(threadIdx.x) / G;
         const bool valid = row < n;
+        CsrQuads<T> q;
+        if (valid) csr_begin(m, row, sub, G, q);
         T s;
-        if (G <= 32) s = csr_group_sum(m, row, valid, sub, G, xa);
-        else s = csr_block_sum(m, row, valid, sub, G, xa);
+        if (G <= 32) s = csr_group_sum(m, q, valid, G, xa);
+        else s = csr_block_sum(m, q, valid, sub, G, xa);
         if (valid && sub == 0) f(row, s);
     }
 }

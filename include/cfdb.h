@@ -431,8 +431,8 @@ typedef struct {
     int fuse_first;   /* first two smoothing sweeps in one kernel, default 0 */
     int sell_rows;    /* rows per CTA of SELL operators (one row per thread per pass): a multiple
                          of 256, default 256 */
-    int krylov_pair;  /* level-0 Krylov SpMV kernels take two rows per thread per pass (1) or one
-                         (0), default 1 */
+    int krylov_pair;  /* level-0 Krylov SpMV kernels load a thread's next row while they sum the current
+                         one (1, default), or take one row at a time (0) */
     int tail_rows;    /* coarse levels of at most this many rows, with all coarser ones, run as one
                          persistent kernel; 0 (default) disables it */
     int col16;        /* FP32 operators keep 16-bit column offsets from a per-slice / per-row base
@@ -453,8 +453,8 @@ typedef struct {
     int tail_cluster; /* with tail_rows: run the tail as one thread-block cluster of this many CTAs
                          (2..16), its phases separated by the hardware cluster barrier; 0
                          (default): a cooperative grid with the bounded grid barrier */
-    int vcycle_pair;  /* V-cycle kernels of SELL operators take two rows per thread per pass (1)
-                         or one (0, default) */
+    int vcycle_pair;  /* V-cycle kernels of SELL operators load a thread's next row while they sum the
+                         current one (1), or take one row at a time (0, default) */
     int krylov_stage; /* level-0 Krylov SpMV with the operator streamed through shared memory by
                          bulk copies, in this many buffers (2..4); 0 (default): loaded by the
                          threads (krylov_pair). Same results bit for bit. */
