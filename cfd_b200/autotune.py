@@ -5,7 +5,7 @@ The knobs are those of `Tuning` (include/cfdb.h, cfdb_tuning):
 * target_tiles - level-0 Krylov tiles (0: 256 rows each; else about this many CTAs),
 * wide_row     - average row length above which a level switches from SELL-32 rows to
                  CSR lane groups,
-* lanes_div    - lanes per CSR row = average row length / lanes_div,
+* lanes_div    - lanes per CSR row = 4 x average row length / lanes_div,
 * fuse_first   - first two Jacobi sweeps of the pre-smoothing fused into one kernel,
 * sell_rows    - rows per CTA of SELL operators (one row per thread per pass),
 * krylov_pair  - level-0 Krylov SpMV kernels load the next row ahead, or take one at a time,

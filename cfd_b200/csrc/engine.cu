@@ -303,25 +303,41 @@ std::vector<double> inverse_diagonal(const HostCsr& a) {
     return d;
 }
 
-int grid_of(long long n) { return static_cast<int>(std::max<long long>(1, (n + 255) / 256)); }
-
-// Kernel launch, with programmatic dependent launch when pdl: the kernel may be scheduled while
-// its predecessor in the stream finishes (every kernel of kernels.cuh starts with pdl_entry(),
-// which lets its own successor be scheduled and then waits for its predecessor's completion).
-template <class... P, class... A>
-void launch_k(bool pdl, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A&&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(grid));
-    cfg.blockDim = dim3(static_cast<unsigned>(block));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    CFDB_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+// Whether an operator takes CSR lane groups instead of SELL rows: rows of more than wide_row
+// entries, and operators with too few rows to fill the GPU with one thread each. Short rows stay
+// in SELL longer: a row of up to 8 entries is one batch of a thread. Measured (FP32 / FP64 us, L2
+// resident, back to back, SELL against the lanes of csr_lanes): 217K rows of 16.8 entries 7.7
+// against 8.6 / 10.3 against 14.5; 146K of 12.8: 3.4 against 5.6 / 4.9 against 9.0; 62.8K of
+// 16.3: 3.4 against 3.3 / 5.0 against 5.0; 51K of 16.7: 4.9 against 2.4 / 6.6 against 4.5; 51K of
+// 6.4: 1.9 against 2.0 / 2.5 against 3.5; 13K of 8.1: 1.7 against 1.6 / 2.2 against 2.1; 4.2K of
+// 6.6: 1.6 against 1.2 / 1.8 against 1.6.
+bool use_lanes(double rows, double avg, int wide_row) {
+    if (rows <= 0) return false;
+    if (avg > wide_row) return true;
+    return rows < (avg <= 8.0 ? 16384.0 : 98304.0);
 }
+
+// Lanes per CSR row (a power of two, 4..256): doubled while a lane would take more than one quad of
+// the row (lanes_div 16; in proportion otherwise) and the operator's threads stay within one
+// resident wave (148 x 2048 in FP32; half of that in FP64 and for rows of several warps, whose
+// block sums cost two block barriers); rows of more than two passes may take a second wave.
+// Measured (FP32 us by lanes 4 / 8 / 16 / 32 / 64): 514 rows of 25 entries 1.7 / 1.3 / 1.3 / 1.3 /
+// 1.6; 3.8K of 77: 3.2 / 2.5 / 2.3 / 2.1 / 3.3; 13.4K of 139: 13.4 / 5.5 / 4.4 / 5.7 / 8.9; 62.8K of
+// 91.5: 15.0 / 12.1 / 13.4 / 19.6 / 33.9; 1.0K of 350: 17.0 / 9.1 / 5.4 / 3.7 / 3.0 (128: 2.5).
+int csr_lanes(double rows, double avg, int lanes_div, bool fp64) {
+    constexpr double kWave = 148.0 * 2048.0;
+    int lanes = 4;
+    while (lanes < 256 && 0.25 * lanes * std::max(lanes_div, 1) < avg) {
+        const double threads = 2.0 * lanes * rows;
+        const bool one_wave = threads <= (fp64 || lanes >= 32 ? 0.5 * kWave : kWave);
+        const bool two_waves = lanes < 32 && avg > 16.0 * lanes && threads <= 2.0 * kWave;
+        if (!one_wave && !two_waves) break;
+        lanes *= 2;
+    }
+    return lanes;
+}
+
+int grid_of(long long n) { return static_cast<int>(std::max<long long>(1, (n + 255) / 256)); }
 
 } // namespace
 
@@ -488,9 +504,7 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
     // Launch tiles of one operator over the rows of `row_level` of the systems `include`
     // selects (a prefix in batch order); `nc` marks the systems that continue past that level.
     auto op_tiles = [&](DevSell64_32& m, int fmt, int row_level, auto include, auto nc) {
-        const int rpt = fmt == kFmtSell ? std::max(kSellRows, tuning_.sell_rows / kSellRows * kSellRows)
-                                        : (fmt <= 32 ? kFineRows : kBlock / fmt);
-        m.block = fmt == kFmtSell ? kBlock : (fmt <= 32 ? kFineRows * fmt : kBlock);
+        const int rpt = fmt == kFmtSell ? std::max(kSellRows, tuning_.sell_rows / kSellRows * kSellRows) : kBlock / fmt;
         std::vector<int> trow, tsys;
         int n_nc = -1, end = 0;
         for (int k = 0; k < n_sys_; ++k) {
@@ -635,20 +649,9 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
                 nnz += dsrc != nullptr ? dsrc->nnz : pick(s).nnz();
                 rows += pick(s).n_rows;
             }
-            // lanes per row: about lanes_div entries per lane, and enough lanes in all to keep
-            // ~150K threads busy on operators with few, long rows; never more than the row length
             const double avg = rows > 0 ? static_cast<double>(nnz) / static_cast<double>(rows) : 0.0;
-            constexpr double kFillThreads = 148.0 * 1024.0;
-            int lanes = 4;
-            while (lanes < 256 && 2.0 * lanes <= std::max(avg, 4.0) &&
-                   (lanes * std::max(tuning_.lanes_div, 1) < avg ||
-                    static_cast<double>(lanes) * static_cast<double>(rows) < kFillThreads)) {
-                lanes *= 2;
-            }
-            // CSR lane groups for long rows, and for operators too short to fill the GPU with one
-            // thread per row; SELL (rows sorted by length within 256-row windows) otherwise
-            const bool wide = !ordered_ && rows > 0 &&
-                              (avg > tuning_.wide_row || static_cast<double>(rows) < kFillThreads);
+            const bool wide = !ordered_ && use_lanes(static_cast<double>(rows), avg, tuning_.wide_row);
+            const int lanes = csr_lanes(static_cast<double>(rows), avg, tuning_.lanes_div, need64_);
             if (dsrc != nullptr) {
                 // the same layouts built on the device (columns offset 0: one system)
                 const DevCsr& a = *dsrc;
@@ -1314,11 +1317,10 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
     struct Launch {
         Tiles first;
         int second; // grid
-        int block;
         int visit;  // row-visiting strategy of the operator's kernels
     };
     auto TL = [&](int, const DevSell64_32& m, bool nc) -> Launch {
-        return {m.tiles, nc ? m.n_tiles_nc : m.n_tiles, m.block, vcycle_visit(m)};
+        return {m.tiles, nc ? m.n_tiles_nc : m.n_tiles, vcycle_visit(m)};
     };
     std::vector<T*> cur(L, nullptr);
     // levels lt and below run in the persistent tail kernel when its phases are prepared
@@ -1343,8 +1345,8 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
             T* c = start;
             for (int k = 1; k < sweeps_; ++k) {
                 T* o = c == x ? y : x;
-                if (l == 0) with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, ta.block, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
-                else with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, ta.block, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
+                if (l == 0) with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
+                else with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
                 mark("smooth", l, spmv_b(d.a, n, n) + sv * n + sb * n);
                 c = o;
             }
@@ -1352,30 +1354,30 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
         } else {
             const auto ta = TL(l, d.a, true);
             if (l == 0) {
-                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_first<T, double, decltype(V)::value>, ta.second, ta.block, 0, s, A(l), ta.first, stv, WD(l), r_, start, fuse); });
+                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_first<T, double, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), r_, start, fuse); });
             } else {
-                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_first<T, T, decltype(V)::value>, ta.second, ta.block, 0, s, A(l), ta.first, stv, WD(l), Bv(l), start, fuse); });
+                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_first<T, T, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), Bv(l), start, fuse); });
             }
             mark("smooth_first", l, fuse ? spmv_b(d.a, n, n) - sv * n + sv * n + sb * n : 2.0 * sv * n + sb * n);
             T* c = start;
             for (int k = fuse ? 2 : 1; k < sweeps_; ++k) {
                 T* o = c == x ? y : x;
-                if (l == 0) with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, ta.block, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
-                else with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, ta.block, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
+                if (l == 0) with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
+                else with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
                 mark("smooth", l, spmv_b(d.a, n, n) + sv * n + sb * n);
                 c = o;
             }
             cur[l] = c;
         }
         const auto tr = TL(l, d.a, true);
-        if (l == 0) with_visit(tr.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_residual<T, double, decltype(V)::value>, tr.second, tr.block, 0, s, A(l), tr.first, stv, r_, cur[l], Tv(l)); });
-        else with_visit(tr.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_residual<T, T, decltype(V)::value>, tr.second, tr.block, 0, s, A(l), tr.first, stv, Bv(l), cur[l], Tv(l)); });
+        if (l == 0) with_visit(tr.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_residual<T, double, decltype(V)::value>, tr.second, kBlock, 0, s, A(l), tr.first, stv, r_, cur[l], Tv(l)); });
+        else with_visit(tr.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_residual<T, T, decltype(V)::value>, tr.second, kBlock, 0, s, A(l), tr.first, stv, Bv(l), cur[l], Tv(l)); });
         mark("residual", l, spmv_b(d.a, n, n) + sb * n);
         const DevLevel& nx = lv_[l + 1];
         const auto tq = TL(l + 1, d.r, false);
         const bool next_x1 = x1_by_restrict && l + 2 < L && nx.n_rows_nc > 0;
         with_visit(tq.visit, [&](auto V) {
-            launch_k(tuning_.pdl != 0, k_vc_spmv<T, decltype(V)::value>, tq.second, tq.block, 0, s, 
+            launch_k(tuning_.pdl != 0, k_vc_spmv<T, decltype(V)::value>, tq.second, kBlock, 0, s, 
                 R(l), tq.first, stv, Tv(l), Bv(l + 1), next_x1 ? WD(l + 1) : nullptr,
                 next_x1 ? start_buffer<T>(l + 1) : nullptr, next_x1 ? nx.n_rows_nc : 0);
         });
@@ -1408,7 +1410,7 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
         T* c = cur[l];
         const auto tp = TL(l, d.p, true);
         with_visit(tp.visit, [&](auto V) {
-            launch_k(tuning_.pdl != 0, k_vc_prolong<T, decltype(V)::value>, tp.second, tp.block, 0, s, P(l), tp.first, stv, X(l + 1), c);
+            launch_k(tuning_.pdl != 0, k_vc_prolong<T, decltype(V)::value>, tp.second, kBlock, 0, s, P(l), tp.first, stv, X(l + 1), c);
         });
         const auto ta = TL(l, d.a, true);
         mark("prolong", l, spmv_b(d.p, n, lv_[l + 1].n_rows) + sv * n);
@@ -1422,10 +1424,10 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
                 });
                 mark("smooth_dot", l, spmv_b(d.a, n, n) + sv * n + sb * n + (flexible ? 8.0 * n : 0.0));
             } else if (l == 0) {
-                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, ta.block, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
+                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
                 mark("smooth", l, spmv_b(d.a, n, n) + sv * n + sb * n);
             } else {
-                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, ta.block, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
+                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
                 mark("smooth", l, spmv_b(d.a, n, n) + sv * n + sb * n);
             }
             c = o;
@@ -1806,12 +1808,12 @@ double Engine::time_sweep(int level, int reps, double* bytes) {
         }
         with_visit(visit, [&](auto V) {
             if (level == 0) {
-                launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, grid, m.block, 0, stream_, op, tiles, nullptr, wd, r_, x, y);
+                launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, grid, kBlock, 0, stream_, op, tiles, nullptr, wd, r_, x, y);
             } else {
                 const T* bv;
                 if constexpr (sizeof(T) == 8) bv = d.b64;
                 else bv = d.b32;
-                launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, grid, m.block, 0, stream_, op, tiles, nullptr, wd, bv, x, y);
+                launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, grid, kBlock, 0, stream_, op, tiles, nullptr, wd, bv, x, y);
             }
         });
     };

@@ -4,6 +4,7 @@
 #pragma once
 
 #include <memory>
+#include <utility>
 #include <vector>
 
 #include "common.hpp"
@@ -39,8 +40,8 @@ struct SystemSpec {
 struct Tuning {
     int target_tiles = 148 * 8; // level-0 Krylov tiles: about this many (0: 256 rows each)
     int wide_row = 48;          // average row length above which CSR lane groups are used
-    int lanes_div = 16;         // lanes per CSR row ~ average row length / lanes_div (4..256),
-                                // and at least enough lanes to give ~150K threads per operator
+    int lanes_div = 16;         // lanes per CSR row ~ 4 x average row length / lanes_div (4..256),
+                                // within a wave of threads per operator
     int fuse_first = 0;         // first two smoothing sweeps in one kernel (x1 recomputed)
     int sell_rows = kSellRows;  // rows per CTA of SELL operators (multiple of kSellRows)
     int krylov_pair = 1;        // level-0 Krylov SpMV kernels: the next row's operands loaded while
@@ -59,6 +60,24 @@ struct Tuning {
     int krylov_stage = 0;       // level-0 Krylov SpMV with the operator staged through shared
                                 // memory in this many buffers (2..4); 0: krylov_pair's kernels
 };
+
+// Kernel launch, with programmatic dependent launch when pdl: the kernel may be scheduled while
+// its predecessor in the stream finishes (every such kernel lets its own successor be scheduled
+// and waits for its predecessor's completion: pdl_launch / pdl_wait in kernels.cuh).
+template <class... P, class... A>
+void launch_k(bool pdl, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    CFDB_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+}
 
 struct SolveRequest {
     double tol = 1e-10;
@@ -165,12 +184,11 @@ private:
         long long slots = 0;  // stored entries (SELL: with padding)
         long long nnz = 0;    // algorithmic nonzeros
         int max8_slots = 0;   // SELL: most slots of any 8 consecutive slices (a staged chunk)
-        // launch tiles of the operator's own row space: kSellRows rows (SELL), 8 rows (CSR,
-        // G <= 32) or 256 / G rows (CSR, G > 32); block = threads per CTA
+        // launch tiles of the operator's own row space, 256 threads each: sell_rows rows (SELL) or
+        // 256 / G rows (CSR)
         Tiles tiles{};
         int n_tiles = 0;
         int n_tiles_nc = 0;   // tiles of systems that continue to a coarser level
-        int block = kBlock;
     };
     struct DevLevel {
         int n_rows = 0;     // all present systems (padded)

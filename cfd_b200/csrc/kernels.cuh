@@ -48,11 +48,12 @@ __device__ __forceinline__ void pdl_entry() {
 //  0 (kFmtSell): SELL-32, one thread per row; `slice` = slice offsets. Row sums keep the CSR
 //     order.
 //  G in {4, 8, 16, 32, 64, 128, 256}: CSR with G lanes per row; `slice` = row offsets. Used
-//     for wide coarse-level rows (tens to thousands of entries), where one thread per row would
-//     serialise long load chains; lanes sum strided entries and combine them with a fixed
+//     for wide coarse-level rows (tens to thousands of entries) and for operators of few rows,
+//     where one thread per row would serialise long load chains; lanes sum strided entries and combine them with a fixed
 //     butterfly (and, above 32 lanes, a fixed-order sum over the row's warps): deterministic,
-//     but not the sequential CSR order. Tiles of a CSR operator hold 8 rows (G <= 32, blockDim
-//     8 G) or 256 / G rows (G > 32, blockDim 256).
+//     but not the sequential CSR order. Tiles of a CSR operator hold 256 / G rows (8-row tiles
+//     of 8 G threads took 28 us instead of 8.5 us on 217K rows of 17 entries with G = 4: CTAs of
+//     one warp fill half of an SM's warp slots).
 enum : int { kFmtSell = 0 };
 
 template <class T> struct Sell {
@@ -410,11 +411,6 @@ __device__ __forceinline__ T csr_block_sum(const Sell<T>& m, CsrQuads<T>& q, boo
     return t;
 }
 
-// Rows of a fine tile (CSR operators with G <= 32): one group of G = fmt lanes per row,
-// blockDim = 8 * G. Wider groups take 256 / G rows per tile with blockDim 256.
-constexpr int kFineRows = 8;
-
-
 // Row-visiting strategies of the tiled kernels, fixed at compile time so that each kernel
 // instance holds the registers of one strategy only:
 //  kVisitSell4/5/7  SELL, one row per thread per pass, the row's first 4, 5 or 7 entries taken in
@@ -423,7 +419,7 @@ constexpr int kFineRows = 8;
 //                   rows and too few of them to fill the GPU several times over;
 //  kVisitStream5/7  SELL, batches of 5 or 7, the next row's operands loaded while the current row
 //                   is summed (tiles of many rows per thread: the level-0 Krylov kernels);
-//  kVisitWarp       CSR, G <= 32 lanes per row (8 rows per tile);
+//  kVisitWarp       CSR, G <= 32 lanes per row (256 / G rows per tile);
 //  kVisitBlock      CSR, G = 64..256 lanes per row (256 / G rows per tile).
 // Every strategy of an operator's format sums each row in the same order.
 enum : int {
@@ -544,16 +540,19 @@ constexpr int kMinBlocks = sizeof(T) == 4
                                                        : 4);
 
 // Strategy of an operator's V-cycle kernels. `width`: stored entries per SELL row; `tiles`: its
-// CTAs. The batch is the narrowest that holds a typical row; rows beyond 8 entries take batches
-// of 7 (FP32) or 4 (FP64) while the operator gives every SM more than two rounds of the long form's
-// four CTAs, and the long form below that.
+// CTAs. The batch is the narrowest that holds a typical row. Rows beyond 8 entries take the long
+// form while its four CTAs per SM hold the operator in one wave (FP64) or two (FP32), and
+// beyond that batches of 7 or, for large FP64 operators, of 4 at full occupancy. Measured
+// (residual, us): 571 tiles of 40 entries FP32 7.9 long against 12.1 by 7, FP64 13.4 against 19.7;
+// 850 tiles of 21 entries FP32 7.7 against 7.8, FP64 12.2 against 9.2; 3365 tiles of 21 entries
+// FP32 34.7 against 30.8, FP64 49.7 against 53.7 (by 4: 44.6).
 __host__ __device__ inline int visit_of(int fmt, double width, int tiles, bool fp64) {
     if (fmt != kFmtSell) return fmt <= 32 ? kVisitWarp : kVisitBlock;
     if (width <= 4.0) return kVisitSell4;
     if (width <= 5.25) return kVisitSell5;
     if (width <= 8.0) return kVisitSell7;
-    if (tiles <= 2 * 4 * 148) return kVisitSellLong;
-    return fp64 ? kVisitSell4 : kVisitSell7;
+    if (tiles <= 148 * (fp64 ? 4 : 8)) return kVisitSellLong;
+    return fp64 && tiles > 148 * 6 ? kVisitSell4 : kVisitSell7;
 }
 
 // Strategy of the level-0 Krylov kernels (FP64 operands, big tiles): the stream forms, or the

@@ -426,8 +426,8 @@ typedef struct {
     int target_tiles; /* level-0 Krylov tiles (reductions): about this many CTAs, default 1184 =
                          148 SMs x 8; 0 = 256 rows per CTA */
     int wide_row;     /* average row length above which CSR lane groups are used, default 48 */
-    int lanes_div;    /* lanes per CSR row ~ average row length / lanes_div (4..256, and enough
-                         lanes for ~150K threads per operator), default 16 */
+    int lanes_div;    /* lanes per CSR row ~ 4 x average row length / lanes_div (4..256, within about a
+                         wave of threads per operator), default 16 */
     int fuse_first;   /* first two smoothing sweeps in one kernel, default 0 */
     int sell_rows;    /* rows per CTA of SELL operators (one row per thread per pass): a multiple
                          of 256, default 256 */
