@@ -821,7 +821,7 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
         vs_ = arena_.alloc<double>(std::max(vs_total_, 1));
         st_ = arena_.alloc<SysState>(n_sys_);
         CFDB_CUDA(cudaMemsetAsync(st_, 0, sizeof(SysState) * n_sys_, st));
-        // two-level reduction: groups of kGroupTiles tiles within each system
+        // reduction groups: kGroupTiles tiles within each system
         std::vector<int> grp0(n_sys_ + 1, 0);
         for (int k = 0; k < n_sys_; ++k) grp0[k + 1] = grp0[k] + ceil_div(sys_tile0[k + 1] - sys_tile0[k], kGroupTiles);
         const int n_groups = std::max(grp0[n_sys_], 1);

@@ -137,11 +137,15 @@ __device__ __forceinline__ void block_sum2(double& a, double& b) {
     __syncthreads();
 }
 
-// Per-tile partial sums and their tickets, reduced in two fixed-order levels: the last CTA of
-// each group of kGroupTiles consecutive tiles of a system sums the group's partials, and the
-// last group of the system sums the group totals. Deterministic, and no CTA sums more than
-// kGroupTiles or (tiles / kGroupTiles) values.
-constexpr int kGroupTiles = 64;
+// Per-tile partial sums and their tickets, reduced in fixed order: the last CTA of each group of
+// kGroupTiles consecutive tiles of a system sums the group's partials, and where a system has more
+// than one group, its last group sums the group totals. Deterministic. A group holds every tile of
+// a system up to a few waves of CTAs, so that a dot product usually costs one ticket and one sum of
+// at most kGroupTiles / 256 pairs a thread: what bounds these tails is the chain of fence, ticket
+// and loads after the last tile, not the sums. With groups of 64 tiles (two chains for systems
+// of more than 16K cells) and full fences, q = A p with its dot took 12.3 us against 8.1 us for a
+// residual on the 32^3 cavity (128 tiles).
+constexpr int kGroupTiles = 2048;
 struct Reduce {
     double* partials;        // 2 per tile
     double* gpartials;       // 2 per group
@@ -151,15 +155,43 @@ struct Reduce {
     const int* grp0;         // n_systems + 1: first group of each system
 };
 
-// Sum of the pairs src[first..last) in index order by the block; valid in thread 0.
+// Sum of the pairs src[first..last) in a fixed order by the block; valid in thread 0. Up to 32 pairs
+// are added one after another by the first warp (no block barriers); more are summed per thread,
+// four 16-byte loads in flight, and then over the block.
 __device__ __forceinline__ void sum_pairs(const double* src, int first, int last, double& a, double& b) {
     a = 0.0;
     b = 0.0;
-    for (int t = first + threadIdx.x; t < last; t += blockDim.x) {
-        a += __ldcg(&src[2 * t]);
-        b += __ldcg(&src[2 * t + 1]);
+    const double2* p = reinterpret_cast<const double2*>(src);
+    const int n = last - first;
+    if (n <= 32) {
+        if (threadIdx.x >= 32) return;
+        const int lane = static_cast<int>(threadIdx.x);
+        const double2 v = lane < n ? __ldcg(&p[first + lane]) : make_double2(0.0, 0.0);
+        for (int i = 0; i < n; ++i) {
+            a += __shfl_sync(0xffffffffu, v.x, i);
+            b += __shfl_sync(0xffffffffu, v.y, i);
+        }
+        return;
+    }
+    for (int t = first + static_cast<int>(threadIdx.x); t < last; t += 4 * kBlock) {
+        double2 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = t + u * kBlock < last ? __ldcg(&p[t + u * kBlock]) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            a += v[u].x;
+            b += v[u].y;
+        }
     }
     block_sum2(a, b);
+}
+
+// Ticket of a finished tile or group: releases this thread's earlier writes and acquires those of
+// the tickets before it (the block barrier that follows extends both to the block).
+__device__ __forceinline__ int take_ticket(int* counter) {
+    int t;
+    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(t) : "l"(counter) : "memory");
+    return t;
 }
 
 // Writes this tile's partials; returns true in every thread of the system's last CTA, whose
@@ -175,27 +207,22 @@ __device__ __forceinline__ bool reduce_system(double& a, double& b, int tile, in
     if (threadIdx.x == 0) {
         r.partials[2 * tile] = a;
         r.partials[2 * tile + 1] = b;
-        __threadfence();
-        const int ticket = atomicAdd(&r.gcounters[gi], 1);
-        last = ticket == gl - gf - 1;
+        last = take_ticket(&r.gcounters[gi]) == gl - gf - 1;
         if (last) r.gcounters[gi] = 0;
     }
     __syncthreads();
     if (!last) return false;
-    __threadfence();
     sum_pairs(r.partials, gf, gl, a, b);
+    const int n_groups = r.grp0[s + 1] - r.grp0[s];
+    if (n_groups == 1) return true;
     if (threadIdx.x == 0) {
         r.gpartials[2 * gi] = a;
         r.gpartials[2 * gi + 1] = b;
-        __threadfence();
-        const int n_groups = r.grp0[s + 1] - r.grp0[s];
-        const int ticket = atomicAdd(&r.counters[s], 1);
-        last = ticket == n_groups - 1;
+        last = take_ticket(&r.counters[s]) == n_groups - 1;
         if (last) r.counters[s] = 0;
     }
     __syncthreads();
     if (!last) return false;
-    __threadfence();
     sum_pairs(r.gpartials, r.grp0[s], r.grp0[s + 1], a, b);
     return true;
 }
