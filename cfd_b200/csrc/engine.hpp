@@ -3,6 +3,7 @@
 // and the captured CUDA graphs of the iteration.
 #pragma once
 
+#include <functional>
 #include <memory>
 #include <utility>
 #include <vector>
@@ -99,6 +100,8 @@ struct SolveResult {
     double true_residual = 0.0;
 };
 
+struct BcgState; // bicgstab.cu
+
 class Engine {
 public:
     explicit Engine(int device);
@@ -152,7 +155,7 @@ public:
     // of one sweep (operator, weights, right-hand side, iterate in and out).
     double time_sweep(int level, int reps, double* bytes);
 
-    // Runs the initial preconditioning and one full iteration eagerly with CUDA events around
+    // Runs the initial residual and one full iteration eagerly with CUDA events around
     // every kernel (all systems kept active); returns per-kernel device time averaged over reps
     // (the first repetition is a warm-up when reps > 1) with the algorithmic bytes of each.
     std::vector<ProfRecord> profile(Mode mode, int reps);
@@ -230,9 +233,23 @@ private:
     }
     // where the residual producers of `mode` write the level-0 first sweep (n = 0: nowhere)
     X1Out x1_out(Mode mode) const;
+    // pieces of a solve: the initial residual; one iteration (preconditioning of the residual, then
+    // the CG step); the FP64 check of the systems that mixed precision brought to the target
     void enqueue_init(Mode mode);
+    void enqueue_precond(Mode mode);
     void enqueue_iteration(Mode mode);
+    void enqueue_true_check();
     void enqueue_rz(Mode mode, int flexible);
+    void enqueue_publish();
+    // captures enqueue() into a graph slot (nothing when it is filled)
+    enum GraphPiece { kInit = 0, kIterate = 1, kVerify = 2 };
+    static constexpr int kBcgGraphs = 3; // graph row of BiCGStab (the first three: the modes)
+    void capture(int row, GraphPiece piece, const std::function<void()>& enqueue);
+    void launch_graph(int row, GraphPiece piece);
+    // launches iterations until no system is active, an error is flagged or `cap` are launched
+    void iterate(int row, int cap);
+    Progress wait_progress(int seq);
+    [[noreturn]] void fail_wait(int error);
     void mark(const char* name, int level, double bytes);
     void release_graphs();
 
@@ -268,14 +285,19 @@ private:
     double* vs_ = nullptr;
     double* dinv0_ = nullptr;
     double* bcg_ = nullptr;  // BiCGStab work vectors (allocated on first use)
+    BcgState* bcg_st_ = nullptr;
+    void enqueue_bicgstab(bool init);
     // Krylov vectors (level 0)
     double *b_ = nullptr, *x_ = nullptr, *r_ = nullptr, *p_ = nullptr, *q_ = nullptr;
     // state
     SysState* st_ = nullptr;
     Reduce red_{};
-    int* n_active_ = nullptr;
+    int* n_active_ = nullptr; // behind the systems' states: one upload starts a solve
     int* error_ = nullptr;
-    int* h_pinned_ = nullptr; // [0] n_active, [1] error
+    int* seq_ = nullptr;           // device count of published records
+    Progress* progress_ = nullptr; // page-locked, mapped: the last record
+    int published_ = 0;            // records published by the work launched so far
+    PinnedBuffer h_state_;         // page-locked image of the states and the two words behind them
     // coarse blocks
     int n_blocks_ = 0;
     int n_single_ = 0;        // systems whose hierarchy has one level (Jacobi-preconditioned CG)
@@ -295,9 +317,9 @@ private:
     float** b_level32_ = nullptr;
     float** x_level32_ = nullptr;
     size_t coarse_smem64_ = 0, coarse_smem32_ = 0;
-    // graphs per mode: [mode][0] init, [mode][1] iteration
-    cudaGraphExec_t graphs_[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
-    int graph_kernels_[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+    // graphs per mode and of BiCGStab, by piece
+    cudaGraphExec_t graphs_[kBcgGraphs + 1][3] = {};
+    int graph_kernels_[kBcgGraphs + 1][3] = {};
     unsigned long long launches_ = 0;
     PhaseTimes build_times_;
     // level-0 layout kept across builds of a single-system plan over the same pattern

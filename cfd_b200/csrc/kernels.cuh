@@ -83,7 +83,7 @@ struct SysState {
     double pq;        // p . q
     double alpha;
     double beta;
-    double true_res;  // |b - A x|_2 recomputed after the solve
+    double true_res;  // |b - A x|_2 recomputed after the solve (negative: not computed)
     int it;           // current iteration number (1-based, as the reference loop counter)
     int max_it;
     int iters_out;    // reported iterations
@@ -91,7 +91,8 @@ struct SysState {
     int converged;
     int first;        // next p-update is p = z
     int phase;        // 0: initial preconditioning, 1: inside the loop
-    int check;        // mixed precision: recursive residual met the target, verify in FP64
+    int check;        // mixed precision: recursive residual met the target (the system rests until
+                      // k_cg_true_check has verified it in FP64)
     int breakdown;    // p.q == 0 or rho == 0 style exits
     int jacobi;       // single-level hierarchy: Jacobi-preconditioned FP64 CG (z = r / diag), as
                       // ldu_matrix.cpp:357 solves a system whose hierarchy has one level
@@ -101,6 +102,15 @@ struct Control {
     int* n_active;   // number of active systems (device)
     int* error;      // device error flag (bounded waits)
     int wait_polls = 1 << 22; // poll limit of the bounded waits (< 0: give up at once)
+};
+
+// Progress of a solve as the host sees it, in page-locked host memory: k_publish writes one record
+// at the end of every iteration, so that the host follows the solve without copies between
+// the iterations on the stream.
+struct Progress {
+    int n_active;
+    int error;
+    int seq; // records published so far (written last)
 };
 
 // Polls allowed to drain a CTA's own bulk copy after its bounded wait expired: the CTA must
@@ -1282,27 +1292,29 @@ static __global__ void __launch_bounds__(kBlock, (X1 == 0 ? 5 : 4)) k_cg_xr(Tile
             } else {
                 s.converged = 1;
                 s.iters_out = s.it;
-                deactivate(s, ctl);
             }
+            deactivate(s, ctl);
         }
     }
 }
 
-// Mixed precision: for systems whose recursive residual met the target, recompute
-// r = b - A x in FP64; converged if |r| <= tol, else restart the search direction.
+// Mixed precision, once no system iterates any more: for the systems whose recursive residual met
+// the target, recompute r = b - A x in FP64; converged if |r| <= tol, else the system iterates
+// again with a new search direction. (Launched in every iteration instead, it was an empty
+// kernel in all but the last: 1 of 17 launches on a 16^3 box.)
 template <int V>
 static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>)) k_cg_true_check(Sell<double> a, Tiles tiles, SysState* st,
                                                           const double* __restrict__ b,
                                                           const double* __restrict__ x,
                                                           double* __restrict__ r, Reduce red,
                                                           Control ctl, X1Out x1o) {
-    pdl_entry();
-    TileCtx c;
-    if (!tile_begin(tiles, st, c)) return;
-    if (st[c.s].check == 0) return;
-    double rr = 0.0, unused = 0.0;
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
     Visit<V, double> vis;
     vis.begin(a, c.r0, c.r1);
+    pdl_wait();
+    if (*((volatile const int*)&st[c.s].check) == 0) return;
+    double rr = 0.0, unused = 0.0;
     vis.run(a, c.r0, c.r1, [x](int j) { return x[j]; }, [&](int row) { return b[row]; },
                     [&](int row, double ax, double bi) {
                         const double ri = __dsub_rn(bi, ax);
@@ -1314,14 +1326,28 @@ static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>))
         SysState& s = st[c.s];
         s.check = 0;
         s.res = sqrt(rr);
+        s.true_res = s.res;
         if (s.res <= s.tol) {
             s.converged = 1;
             s.iters_out = s.it;
-            deactivate(s, ctl);
         } else {
             s.first = 1;
+            s.active = 1;
+            atomicAdd(ctl.n_active, 1);
         }
     }
+}
+
+// The record of one iteration for the host (one thread; the last kernel of its graph).
+static __global__ void k_publish(const int* n_active, const int* error, int* seq, Progress* host) {
+    pdl_entry();
+    const int k = *seq + 1;
+    *seq = k;
+    volatile Progress* h = host;
+    h->n_active = *n_active;
+    h->error = *error;
+    __threadfence_system();
+    h->seq = k;
 }
 
 // Scalar tail of the preconditioning step for one system (last CTA, thread 0):
