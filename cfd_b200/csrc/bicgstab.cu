@@ -256,6 +256,12 @@ static __global__ void __launch_bounds__(kBlock) k_bcg_xr(Tiles tiles, BcgState*
 
 } // namespace
 
+// fn with the stream strategy of the level-0 operator.
+template <class Fn> void Engine::with_krylov(Fn&& fn) const {
+    if (krylov_visit_of(row_width(lv_[0].a), true) == kVisitStream5) fn(std::integral_constant<int, kVisitStream5>{});
+    else fn(std::integral_constant<int, kVisitStream7>{});
+}
+
 // The initial residual, or the five kernels of one iteration.
 void Engine::enqueue_bicgstab(bool init) {
     const DevLevel& d = lv_[0];
@@ -280,11 +286,10 @@ void Engine::enqueue_bicgstab(bool init) {
         launch_k(pdl, k_bcg_spmv<kV, true>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, bcg_st_, sh, s, t, red_, n_active_);
         launch_k(pdl, k_bcg_xr, d.n_tiles, kBlock, 0, stream_, d.tiles, bcg_st_, ph, sh, s, t, r0, x_, r_, red_, n_active_);
     };
-    if (krylov_visit_of(row_width(d.a), true) == kVisitStream5) run(std::integral_constant<int, kVisitStream5>{});
-    else run(std::integral_constant<int, kVisitStream7>{});
+    with_krylov(run);
 }
 
-SolveResult Engine::solve_bicgstab(const SolveRequest& rq) {
+SolveResult Engine::solve_bicgstab(const SolveRequest& rq, bool want_true) {
     CFDB_CUDA(cudaSetDevice(device_));
     if (n_sys_ != 1) fail(1, "solve_bicgstab: single-system plans only");
     const DevLevel& d = lv_[0];
@@ -314,16 +319,18 @@ SolveResult Engine::solve_bicgstab(const SolveRequest& rq) {
     CFDB_CUDA(cudaMemcpyAsync(n_active_, h->words, 2 * sizeof(int), cudaMemcpyHostToDevice, stream_));
     launch_graph(kBcgGraphs, kInit);
     iterate(kBcgGraphs, std::max(rq.max_it, 0) + 1);
-    // |b - A x| of the returned solution, as the CG paths report it
-    const bool pdl = tuning_.pdl != 0;
-    if (krylov_visit_of(row_width(d.a), true) == kVisitStream5)
-        launch_k(pdl, k_true_residual<kVisitStream5>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, st_, b_, x_, red_);
-    else
-        launch_k(pdl, k_true_residual<kVisitStream7>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, st_, b_, x_, red_);
-    ++launches_;
-    CFDB_CUDA(cudaGetLastError());
+    h->cg.true_res = -1.0;
+    if (want_true) {
+        // |b - A x| of the returned solution, as the CG paths report it
+        with_krylov([&](auto V) {
+            launch_k(tuning_.pdl != 0, k_true_residual<decltype(V)::value>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles,
+                     st_, b_, x_, red_);
+        });
+        ++launches_;
+        CFDB_CUDA(cudaGetLastError());
+        CFDB_CUDA(cudaMemcpyAsync(&h->cg, st_, sizeof(SysState), cudaMemcpyDeviceToHost, stream_));
+    }
     CFDB_CUDA(cudaMemcpyAsync(&h->s, bcg_st_, sizeof(BcgState), cudaMemcpyDeviceToHost, stream_));
-    CFDB_CUDA(cudaMemcpyAsync(&h->cg, st_, sizeof(SysState), cudaMemcpyDeviceToHost, stream_));
     CFDB_CUDA(cudaStreamSynchronize(stream_));
     SolveResult out;
     out.iterations = h->s.active ? rq.max_it : h->s.iters_out;

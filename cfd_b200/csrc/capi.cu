@@ -13,6 +13,7 @@
 #include "dsetup.hpp"
 #include "engine.hpp"
 #include "ldu_solve.hpp"
+#include "system_step.hpp"
 #include "host_algos.hpp"
 
 using namespace cfdb;
@@ -225,10 +226,8 @@ struct cfdb_system {
     // persistent LDU solve (cfdb_system_solve_ldu): AmgCache state and device staging
     int age = 0;               // CG solves since the last hierarchy setup
     bool amg_built = false;    // a setup has run (its hierarchy may have one level)
-    int* d_src = nullptr;      // value map of the pattern entries (pat_arena)
     DeviceArena ldu_arena;
     double* ldu_stage = nullptr; // diag | upper | lower | source | x (host-array calls)
-    double* norm_part = nullptr;
 };
 
 namespace {
@@ -303,7 +302,6 @@ void pattern_on_device(cfdb_system* sys, cudaStream_t st) {
     sys->d_dpos = sys->pat_arena.upload(p.diag_pos, st);
     sys->d_upos = sys->pat_arena.upload(p.upper_pos, st);
     sys->d_lpos = sys->pat_arena.upload(p.lower_pos, st);
-    sys->d_src = sys->pat_arena.upload(sys->src, st);
     CFDB_CUDA(cudaStreamSynchronize(st));
 }
 
@@ -343,23 +341,24 @@ void cell_faces(int n, int nf, const int* own, const int* nei, std::vector<int>&
     }
 }
 
-SolveResult run_single(cfdb_system* s, const double* diag, const double* upper, const double* lower,
-                       const double* b, double* x, int method, int use_amg, const cfdb_control* c, bool dev) {
-    if (c == nullptr) fail(CFDB_ERR_BAD_ARG, "null control");
-    if (method != CFDB_METHOD_CG && method != CFDB_METHOD_BICGSTAB) fail(CFDB_ERR_BAD_ARG, "unknown method");
-    if (diag == nullptr || b == nullptr || x == nullptr || (s->pat.n_faces > 0 && (upper == nullptr || lower == nullptr)))
-        fail(CFDB_ERR_BAD_ARG, "null array");
+// The matrix, the right-hand side and the initial guess into the system's engine.
+void load_system(cfdb_system* s, const double* diag, const double* upper, const double* lower, const double* b,
+                 const double* x, bool dev) {
     ensure_engine(s);
     Engine& e = *s->eng;
     const int n = s->pat.n, nf = s->pat.n_faces;
     if (dev) {
         e.set_values_device(diag, upper, lower, n, n + nf);
     } else {
-        // the caller's arrays are read by the copies before this call returns
+        // the caller's arrays are read by the copies before the call returns
         e.upload_values_ldu(diag, upper, lower, n, nf);
     }
     e.set_rhs(0, b, dev);
     e.set_guess(0, x, dev);
+}
+
+// Solves the loaded system.
+SolveResult solve_loaded(cfdb_system* s, int method, int use_amg, const cfdb_control* c, bool want_true) {
     // krylov_cuda.cu:659-669: with a hierarchy and use_amg the solve is AMG-CG whatever the
     // method; otherwise Jacobi-preconditioned CG or BiCGStab on the FP64 level-0 operator
     Mode mode = Mode::Jacobi;
@@ -367,12 +366,26 @@ SolveResult run_single(cfdb_system* s, const double* diag, const double* upper, 
     SolveRequest rq;
     rq.tol = c->abs_tolerance;
     rq.max_it = c->max_iterations;
-    const auto res = (mode == Mode::Jacobi && method == CFDB_METHOD_BICGSTAB) ? std::vector<SolveResult>{e.solve_bicgstab(rq)}
-                                                                              : e.solve(mode, {rq});
-    e.get_solution(0, x, dev);
-    CFDB_CUDA(cudaStreamSynchronize(e.stream()));
-    return res[0];
+    if (mode == Mode::Jacobi && method == CFDB_METHOD_BICGSTAB) return s->eng->solve_bicgstab(rq, want_true);
+    return s->eng->solve(mode, {rq}, want_true)[0];
 }
+
+SolveResult run_single(cfdb_system* s, const double* diag, const double* upper, const double* lower,
+                       const double* b, double* x, int method, int use_amg, const cfdb_control* c, bool dev) {
+    if (c == nullptr) fail(CFDB_ERR_BAD_ARG, "null control");
+    if (method != CFDB_METHOD_CG && method != CFDB_METHOD_BICGSTAB) fail(CFDB_ERR_BAD_ARG, "unknown method");
+    if (diag == nullptr || b == nullptr || x == nullptr || (s->pat.n_faces > 0 && (upper == nullptr || lower == nullptr)))
+        fail(CFDB_ERR_BAD_ARG, "null array");
+    load_system(s, diag, upper, lower, b, x, dev);
+    const SolveResult res = solve_loaded(s, method, use_amg, c, true);
+    s->eng->get_solution(0, x, dev);
+    CFDB_CUDA(cudaStreamSynchronize(s->eng->stream()));
+    return res;
+}
+
+bool solve_ldu(cfdb_system* sys, const double* diag, const double* upper, const double* lower, const double* source,
+               double* x, const cfdb_ldu_settings& settings, const cfdb_amg_settings* amg, bool same_matrix,
+               cfdb_ldu_result& result);
 
 void put_stats(cfdb_stats* st, const SolveResult& r) {
     if (st == nullptr) return;
@@ -1032,61 +1045,95 @@ int cfdb_system_solve_ldu(cfdb_system* sys, const double* diag, const double* up
             fail(CFDB_ERR_BAD_ARG, "unknown method");
         CFDB_CUDA(cudaSetDevice(sys->device));
         ensure_engine(sys);
+        if (device_arrays) {
+            solve_ldu(sys, diag, upper, lower, source, x, *settings, amg, false, *result);
+            CFDB_CUDA(cudaStreamSynchronize(sys->eng->stream()));
+            return;
+        }
         cudaStream_t st = sys->eng->stream();
-        pattern_on_device(sys, st);
-        if (sys->norm_part == nullptr) sys->norm_part = sys->ldu_arena.alloc<double>(3 * static_cast<size_t>(kLduNormBlocks));
-        const double *dd = diag, *du = upper, *dl = lower, *db = source;
-        double* dx = x;
-        if (!device_arrays) {
-            if (sys->ldu_stage == nullptr)
-                sys->ldu_stage = sys->ldu_arena.alloc<double>(4 * static_cast<size_t>(n) + 2 * static_cast<size_t>(nf));
-            double* s = sys->ldu_stage;
-            auto put = [&](double* dst, const double* src, int cnt) {
-                if (cnt > 0) sys->eng->copier().to_device(dst, src, sizeof(double) * cnt, st);
-            };
-            put(s, diag, n);
-            put(s + n, upper, nf);
-            put(s + n + nf, lower, nf);
-            put(s + n + 2 * nf, source, n);
-            put(s + 2 * n + 2 * nf, x, n);
-            dd = s;
-            du = s + n;
-            dl = s + n + nf;
-            db = s + n + 2 * nf;
-            dx = s + 2 * n + 2 * nf;
-        }
-        const LduDevice m{n, nf, sys->d_rp, sys->d_ci, sys->d_src};
-        // ldu_matrix.cpp:118-125: initial normalised residual; nothing to do below the tolerance
-        const LduNorms n0 = ldu_residual_norms(m, dd, du, dl, db, dx, sys->norm_part, st);
-        constexpr double kSmall = 1e-20; // ldu_matrix.cpp:22
-        *result = cfdb_ldu_result{};
-        result->initial_residual = n0.res / (n0.norm + kSmall);
-        result->final_residual = result->initial_residual;
-        if (result->initial_residual < settings->tolerance) return;
-        // ldu_matrix.cpp:293-301: absolute CG target from the relative and absolute tolerances
-        const double target = std::max(settings->rel_tolerance,
-                                       settings->tolerance / std::max(result->initial_residual, kSmall)) *
-                              std::sqrt(n0.r2);
-        const bool cg = settings->method == CFDB_METHOD_CG;
-        // ldu_matrix.cpp:314-353: (re)build the hierarchy at the first CG solve and after
-        // max_age solves, here on the device from this matrix
-        if (cg && (!sys->amg_built || sys->age >= settings->max_age)) {
-            const int rc = cfdb_system_setup_amg_device(sys, dd, du, dl, amg, 1);
-            if (rc != CFDB_OK) fail(rc, g_last_error);
-            sys->age = 0;
-            sys->amg_built = true;
-            result->amg_rebuilt = 1;
-        }
-        if (cg) ++sys->age;
-        const bool use_amg = cg && sys->h != nullptr;
-        const cfdb_control ctl{std::max(target, 1e-300), settings->max_iterations};
-        const SolveResult r = run_single(sys, dd, du, dl, db, dx, settings->method, use_amg ? 1 : 0, &ctl, true);
-        result->iterations = r.iterations;
-        const LduNorms n1 = ldu_residual_norms(m, dd, du, dl, db, dx, sys->norm_part, st);
-        result->final_residual = n1.res / (n1.norm + kSmall);
-        if (!device_arrays) sys->eng->copier().to_host(x, dx, sizeof(double) * n, st);
+        if (sys->ldu_stage == nullptr)
+            sys->ldu_stage = sys->ldu_arena.alloc<double>(4 * static_cast<size_t>(n) + 2 * static_cast<size_t>(nf));
+        double* s = sys->ldu_stage;
+        auto put = [&](double* dst, const double* src, int cnt) {
+            if (cnt > 0) sys->eng->copier().to_device(dst, src, sizeof(double) * cnt, st);
+        };
+        double *dd = s, *du = s + n, *dl = s + n + nf, *db = s + n + 2 * nf, *dx = s + 2 * n + 2 * nf;
+        put(dd, diag, n);
+        put(du, upper, nf);
+        put(dl, lower, nf);
+        put(db, source, n);
+        put(dx, x, n);
+        if (solve_ldu(sys, dd, du, dl, db, dx, *settings, amg, false, *result))
+            sys->eng->copier().to_host(x, dx, sizeof(double) * n, sys->eng->stream());
     });
 }
+
+} // extern "C"
+
+namespace {
+
+// LduMatrix::solve on device arrays. False when the initial residual was already below the
+// tolerance (x is then untouched). amg: settings of a hierarchy that is due (may be null).
+// same_matrix: the engine holds this matrix.
+bool solve_ldu(cfdb_system* sys, const double* diag, const double* upper, const double* lower, const double* source,
+               double* x, const cfdb_ldu_settings& settings, const cfdb_amg_settings* amg, bool same_matrix,
+               cfdb_ldu_result& result) {
+    if (same_matrix) {
+        sys->eng->set_rhs(0, source, true);
+        sys->eng->set_guess(0, x, true);
+    } else {
+        load_system(sys, diag, upper, lower, source, x, true);
+    }
+    // ldu_matrix.cpp:118-125: initial normalised residual; nothing to do below the tolerance
+    const LduNorms n0 = sys->eng->residual_norms();
+    constexpr double kSmall = 1e-20; // ldu_matrix.cpp:22
+    result = cfdb_ldu_result{};
+    result.initial_residual = n0.res / (n0.norm + kSmall);
+    result.final_residual = result.initial_residual;
+    if (result.initial_residual < settings.tolerance) return false;
+    // ldu_matrix.cpp:293-301: absolute CG target from the relative and absolute tolerances
+    const double target = std::max(settings.rel_tolerance,
+                                   settings.tolerance / std::max(result.initial_residual, kSmall)) *
+                          std::sqrt(n0.r2);
+    const bool cg = settings.method == CFDB_METHOD_CG;
+    // ldu_matrix.cpp:314-353: (re)build the hierarchy at the first CG solve and after
+    // max_age solves, here on the device from this matrix
+    if (cg && (!sys->amg_built || sys->age >= settings.max_age)) {
+        const int rc = cfdb_system_setup_amg_device(sys, diag, upper, lower, amg, 1);
+        if (rc != CFDB_OK) fail(rc, g_last_error);
+        sys->age = 0;
+        sys->amg_built = true;
+        result.amg_rebuilt = 1;
+        load_system(sys, diag, upper, lower, source, x, true); // into the new plan
+    }
+    if (cg) ++sys->age;
+    const bool use_amg = cg && sys->h != nullptr;
+    const cfdb_control ctl{std::max(target, 1e-300), settings.max_iterations};
+    const SolveResult r = solve_loaded(sys, settings.method, use_amg ? 1 : 0, &ctl, false);
+    result.iterations = r.iterations;
+    sys->eng->get_solution(0, x, true);
+    const LduNorms n1 = sys->eng->residual_norms();
+    result.final_residual = n1.res / (n1.norm + kSmall);
+    return true;
+}
+
+} // namespace
+
+namespace cfdb {
+
+void solve_ldu_step(cfdb_system* sys, const double* diag, const double* upper, const double* lower,
+                    const double* source, double* x, const cfdb_ldu_settings& settings, const cfdb_amg_settings& amg,
+                    bool same_matrix, cfdb_ldu_result& result) {
+    if (settings.method != CFDB_METHOD_CG && settings.method != CFDB_METHOD_BICGSTAB)
+        fail(CFDB_ERR_BAD_ARG, "unknown method");
+    CFDB_CUDA(cudaSetDevice(sys->device));
+    ensure_engine(sys);
+    (void)solve_ldu(sys, diag, upper, lower, source, x, settings, &amg, same_matrix, result);
+}
+
+} // namespace cfdb
+
+extern "C" {
 
 int cfdb_system_assemble_device(cfdb_system* sys, const double* flux, const double* gamma, const double* delta,
                                 double convection, double* upper, double* lower, double* diag, double* div) {

@@ -396,6 +396,7 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
     tail_bar_ = nullptr;
     bcg_ = nullptr;
     bcg_st_ = nullptr;
+    norms_ = nullptr;
     n_sys_ = static_cast<int>(systems.size());
     if (n_sys_ == 0) fail(1, "engine: no systems");
     if (sweeps < 0) fail(1, "engine: negative smoothing sweeps");
@@ -939,15 +940,13 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
 void Engine::set_values_device(const double* p0, const double* p1, const double* p2, int n1, int n2) {
     const DevLevel& d = lv_[0];
     ValueSource vs{p0, p1, p2, n1, n2};
-    const long long n = std::max<long long>(d.a.slots, d.n_rows);
+    const long long n = std::max<long long>(ceil_div(static_cast<int>(d.a.slots), kFillSlots), d.n_rows);
+    // dinv0_: the plain inverse diagonal (Jacobi preconditioning)
     launch_k(tuning_.pdl != 0, k_fill_level0, grid_of(n), 256, 0, stream_, static_cast<int>(d.a.slots), d.n_rows, src0_, diag_src0_, vs,
                                                    weight_, d.a.s64.val ? const_cast<double*>(d.a.s64.val) : nullptr,
                                                    d.a.s32.val ? const_cast<float*>(d.a.s32.val) : nullptr, d.wd64,
-                                                   d.wd32);
-    // plain inverse diagonal for Jacobi preconditioning: weight 1
-    launch_k(tuning_.pdl != 0, k_fill_level0, grid_of(d.n_rows), 256, 0, stream_, 0, d.n_rows, src0_, diag_src0_, vs, 1.0, nullptr,
-                                                          nullptr, dinv0_, nullptr);
-    launches_ += 2;
+                                                   d.wd32, dinv0_);
+    ++launches_;
     CFDB_CUDA(cudaGetLastError());
 }
 
@@ -1742,7 +1741,7 @@ void Engine::fail_wait(int error) {
                        : "solve: a bounded device wait expired (coarse-level staging)");
 }
 
-std::vector<SolveResult> Engine::solve(Mode mode, const std::vector<SolveRequest>& req) {
+std::vector<SolveResult> Engine::solve(Mode mode, const std::vector<SolveRequest>& req, bool want_true) {
     CFDB_CUDA(cudaSetDevice(device_));
     if (static_cast<int>(req.size()) != n_sys_) fail(1, "solve: one request per system expected");
     if (mode != Mode::Jacobi && !has_amg_) fail(5, "solve: no AMG hierarchy set");
@@ -1782,7 +1781,7 @@ std::vector<SolveResult> Engine::solve(Mode mode, const std::vector<SolveRequest
     }
     // true residuals for reporting, where the check has not just computed them
     bool missing = false;
-    for (int s = 0; s < n_sys_; ++s) missing = missing || !(hs[s].converged && hs[s].true_res >= 0.0);
+    for (int s = 0; s < n_sys_ && want_true; ++s) missing = missing || !(hs[s].converged && hs[s].true_res >= 0.0);
     if (missing) {
         const DevLevel& d = lv_[0];
         with_krylov_visit(krylov_visit(), [&](auto V) {

@@ -12,6 +12,7 @@
 #include "dsetup.hpp"
 #include "host_algos.hpp"
 #include "kernels.cuh"
+#include "ldu_solve.hpp"
 
 namespace cfdb {
 
@@ -100,7 +101,8 @@ struct SolveResult {
     double true_residual = 0.0;
 };
 
-struct BcgState; // bicgstab.cu
+struct BcgState;  // bicgstab.cu
+struct NormState; // ldu_solve.cu
 
 class Engine {
 public:
@@ -139,10 +141,14 @@ public:
     void set_guess(int s, const double* x, bool device_ptr);
     void get_solution(int s, double* x, bool device_ptr);
 
-    // Runs the solve for all systems on the engine stream; blocks until done.
-    std::vector<SolveResult> solve(Mode mode, const std::vector<SolveRequest>& req);
+    // Runs the solve for all systems on the engine stream; blocks until done. want_true: also
+    // |b - A x| of every solution (without it, only where the solve has computed it).
+    std::vector<SolveResult> solve(Mode mode, const std::vector<SolveRequest>& req, bool want_true = true);
+    // Normalised residual norms of the level-0 system with the current values, right-hand side and
+    // iterate (single-system plans; ldu_solve.cu). Blocks until done.
+    LduNorms residual_norms();
     // Jacobi-preconditioned BiCGStab on the level-0 operator (single-system plans; bicgstab.cu).
-    SolveResult solve_bicgstab(const SolveRequest& req);
+    SolveResult solve_bicgstab(const SolveRequest& req, bool want_true = true);
 
     // Launch the pieces of one V-cycle application z = M^-1 r for system-batch inputs that are
     // already in the level-0 residual vector (used by the parity tests).
@@ -286,7 +292,10 @@ private:
     double* dinv0_ = nullptr;
     double* bcg_ = nullptr;  // BiCGStab work vectors (allocated on first use)
     BcgState* bcg_st_ = nullptr;
+    NormState* norms_ = nullptr; // residual_norms (allocated on first use)
+    Reduce red2_{};
     void enqueue_bicgstab(bool init);
+    template <class Fn> void with_krylov(Fn&& fn) const;
     // Krylov vectors (level 0)
     double *b_ = nullptr, *x_ = nullptr, *r_ = nullptr, *p_ = nullptr, *q_ = nullptr;
     // state

@@ -646,27 +646,40 @@ __device__ __forceinline__ double vs_load(const ValueSource& v, int i) {
     return v.p2[i - v.n2];
 }
 
-// val[s] = source value of slot s; wd[i] = w * (diag_i != 0 ? 1/diag_i : 1)
-// (krylov_cuda.cu:541-562: assemble_diag / assemble_faces / inv_diag kernels, fused).
-static __global__ void k_fill_level0(int n_slots, int n_rows, const int* __restrict__ src,
+// val[s] = source value of slot s; wd[i] = w * (diag_i != 0 ? 1/diag_i : 1) and dinv[i] the same
+// without the weight (krylov_cuda.cu:541-562: assemble_diag / assemble_faces / inv_diag kernels,
+// fused). A thread fills kFillSlots slots, a block's worth apart, so that their map loads and then
+// their gathers are in flight together.
+constexpr int kFillSlots = 4;
+static __global__ void __launch_bounds__(256) k_fill_level0(int n_slots, int n_rows, const int* __restrict__ src,
                               const int* __restrict__ diag_src, ValueSource vs, double weight,
                               double* __restrict__ val64, float* __restrict__ val32,
-                              double* __restrict__ wd64, float* __restrict__ wd32) {
-    pdl_entry();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n_slots) {
-        const int s = __ldg(&src[i]);
-        const double v = s >= 0 ? vs_load(vs, s) : 0.0;
-        if (val64 != nullptr) val64[i] = v;
-        if (val32 != nullptr) val32[i] = static_cast<float>(v);
+                              double* __restrict__ wd64, float* __restrict__ wd32, double* __restrict__ dinv) {
+    pdl_launch();
+    const int i0 = blockIdx.x * 256 * kFillSlots + threadIdx.x;
+    int s[kFillSlots];
+#pragma unroll
+    for (int u = 0; u < kFillSlots; ++u) s[u] = i0 + 256 * u < n_slots ? __ldg(&src[i0 + 256 * u]) : -1;
+    pdl_wait();
+    double v[kFillSlots];
+#pragma unroll
+    for (int u = 0; u < kFillSlots; ++u) v[u] = s[u] >= 0 ? vs_load(vs, s[u]) : 0.0;
+#pragma unroll
+    for (int u = 0; u < kFillSlots; ++u) {
+        const int i = i0 + 256 * u;
+        if (i >= n_slots) continue;
+        if (val64 != nullptr) val64[i] = v[u];
+        if (val32 != nullptr) val32[i] = static_cast<float>(v[u]);
     }
+    const int i = blockIdx.x * 256 + threadIdx.x;
     if (i < n_rows) {
-        const int s = __ldg(&diag_src[i]);
-        const double d = s >= 0 ? vs_load(vs, s) : 0.0;
-        const double dinv = d != 0.0 ? 1.0 / d : 1.0;
-        const double wd = weight * dinv;
+        const int sd = __ldg(&diag_src[i]);
+        const double d = sd >= 0 ? vs_load(vs, sd) : 0.0;
+        const double di = d != 0.0 ? 1.0 / d : 1.0;
+        const double wd = weight * di;
         if (wd64 != nullptr) wd64[i] = wd;
         if (wd32 != nullptr) wd32[i] = static_cast<float>(wd);
+        dinv[i] = di;
     }
 }
 

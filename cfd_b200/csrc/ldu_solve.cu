@@ -1,100 +1,114 @@
-// Residual norms of an LDU system on the device, for the persistent LDU solve
+// Residual norms of an engine's level-0 system, for the persistent LDU solve
 // (LduMatrix::solve_persistent, ldu_matrix.cpp:287-366, and LduMatrix::residual_norms,
 // ldu_matrix.cpp:69-103).
 //
-// Row i of A x is summed over the CSR pattern of the LDU matrix (columns ascending), its
-// coefficients read from [diag | upper | lower] through the pattern's value map. Each block
-// sums a fixed set of rows and the host adds the block sums in block order, so the norms are
-// reproducible; they differ from the reference's face-loop sums only in summation order.
+// Row i of A x is summed over the engine's SELL slots, which hold the LDU matrix's CSR pattern in
+// column order with its values already scattered: coalesced columns and values, where a pass over
+// the CSR pattern with each value fetched through the LDU value map took 44 us per call on the
+// 1.3M-cell tet box (and two host round trips). The mean of x stays on the device between the
+// two kernels. Sums are the tile reductions of the CG kernels: reproducible, and different from the
+// reference's face-loop sums only in summation order.
 #include "ldu_solve.hpp"
 
-#include <vector>
+#include "engine.hpp"
 
 namespace cfdb {
 
+struct NormState {
+    double x_ref;
+    double res, norm, r2;
+};
+
 namespace {
 
-constexpr int kNormThreads = 256;
-
-__device__ __forceinline__ double ldu_value(int s, int n, int nf, const double* __restrict__ diag,
-                                            const double* __restrict__ upper, const double* __restrict__ lower) {
-    return s < n ? diag[s] : s < n + nf ? upper[s - n] : lower[s - n - nf];
-}
-
-template <int K> __device__ void block_sums(double (&v)[K], double* part) {
-    __shared__ double sh[K][kNormThreads / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// x_ref = sum of x over the n user rows / n
+__global__ void __launch_bounds__(kBlock) k_ldu_mean(Tiles tiles, int n, const double* __restrict__ x, Reduce red,
+                                                     NormState* out) {
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    pdl_wait();
+    double s = 0.0, unused = 0.0;
+    for (int r0 = c.r0 + threadIdx.x; r0 < c.r1; r0 += 4 * kBlock) {
+        double v[4];
 #pragma unroll
-    for (int q = 0; q < K; ++q) {
-        double s = v[q];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) sh[q][w] = s;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+        for (int u = 0; u < 4; ++u) v[u] = r0 + u * kBlock < min(c.r1, n) ? x[r0 + u * kBlock] : 0.0;
 #pragma unroll
-        for (int q = 0; q < K; ++q) {
-            double s = 0.0;
-            for (int u = 0; u < kNormThreads / 32; ++u) s += sh[q][u];
-            part[K * blockIdx.x + q] = s;
-        }
+        for (int u = 0; u < 4; ++u) s += v[u];
     }
+    if (reduce_system(s, unused, c.tile, c.s, red) && threadIdx.x == 0) out->x_ref = s / static_cast<double>(n);
 }
 
-__global__ void __launch_bounds__(kNormThreads) k_sum(int n, const double* __restrict__ x, double* part) {
-    double v[1] = {0.0};
-    for (int i = blockIdx.x * kNormThreads + threadIdx.x; i < n; i += gridDim.x * kNormThreads) v[0] += x[i];
-    block_sums<1>(v, part);
-}
-
-// per block: sum |b - Ax|, sum |Ax - rs x_ref| + |b - rs x_ref| (rs = row sum), sum (b - Ax)^2
-__global__ void __launch_bounds__(kNormThreads) k_norms(int n, int nf, const int* __restrict__ rp,
-                                                        const int* __restrict__ ci, const int* __restrict__ src,
-                                                        const double* __restrict__ diag, const double* __restrict__ upper,
-                                                        const double* __restrict__ lower, const double* __restrict__ b,
-                                                        const double* __restrict__ x, double x_ref, double* part) {
-    double v[3] = {0.0, 0.0, 0.0};
-    for (int i = blockIdx.x * kNormThreads + threadIdx.x; i < n; i += gridDim.x * kNormThreads) {
+// sum |b - Ax|, sum |Ax - rs x_ref| + |b - rs x_ref| (rs = row sum), sum (b - Ax)^2 over the n user
+// rows. B: entries of a row taken in one batch.
+template <int B>
+__global__ void __launch_bounds__(kBlock) k_ldu_norms(Sell<double> m, Tiles tiles, int n, const double* __restrict__ b,
+                                                      const double* __restrict__ x, Reduce red, Reduce red2,
+                                                      NormState* out) {
+    pdl_launch();
+    const TileCtx c = tile_of(tiles);
+    pdl_wait();
+    const double x_ref = *reinterpret_cast<volatile const double*>(&out->x_ref);
+    double res = 0.0, norm = 0.0, r2 = 0.0, unused = 0.0;
+    for (int row = c.r0 + threadIdx.x; row < min(c.r1, n); row += kBlock) {
+        SellRow r = sell_row_at(m, row);
+        const double bi = b[row];
         double ax = 0.0, rs = 0.0;
-        for (int k = rp[i]; k < rp[i + 1]; ++k) {
-            const double a = ldu_value(src[k], n, nf, diag, upper, lower);
-            ax += a * x[ci[k]];
-            rs += a;
+        for (; r.k < r.e; r.k += 32 * B) {
+            double v[B], xv[B];
+            int cc[B];
+            sell_load<B>(m, r.k, r.e, 0, v, cc);
+#pragma unroll
+            for (int u = 0; u < B; ++u) xv[u] = cc[u] >= 0 ? x[cc[u]] : 0.0;
+#pragma unroll
+            for (int u = 0; u < B; ++u)
+                if (cc[u] >= 0) {
+                    ax = __dadd_rn(ax, __dmul_rn(v[u], xv[u]));
+                    rs = __dadd_rn(rs, v[u]);
+                }
         }
-        const double ax_ref = rs * x_ref;
-        const double r = b[i] - ax;
-        v[0] += fabs(r);
-        v[1] += fabs(ax - ax_ref) + fabs(b[i] - ax_ref);
-        v[2] += r * r;
+        const double ax_ref = __dmul_rn(rs, x_ref);
+        const double ri = __dsub_rn(bi, ax);
+        res += fabs(ri);
+        norm += fabs(ax - ax_ref) + fabs(bi - ax_ref);
+        r2 += __dmul_rn(ri, ri);
     }
-    block_sums<3>(v, part);
+    if (reduce_system(res, norm, c.tile, c.s, red) && threadIdx.x == 0) {
+        out->res = res;
+        out->norm = norm;
+    }
+    if (reduce_system(r2, unused, c.tile, c.s, red2) && threadIdx.x == 0) out->r2 = r2;
 }
 
 } // namespace
 
-LduNorms ldu_residual_norms(const LduDevice& m, const double* diag, const double* upper, const double* lower,
-                            const double* b, const double* x, double* part, cudaStream_t st) {
-    LduNorms out;
-    if (m.n == 0) return out;
-    std::vector<double> h(3 * static_cast<size_t>(kLduNormBlocks));
-    k_sum<<<kLduNormBlocks, kNormThreads, 0, st>>>(m.n, x, part);
-    CFDB_CUDA(cudaGetLastError());
-    CFDB_CUDA(cudaMemcpyAsync(h.data(), part, sizeof(double) * kLduNormBlocks, cudaMemcpyDeviceToHost, st));
-    CFDB_CUDA(cudaStreamSynchronize(st));
-    double sum = 0.0;
-    for (int q = 0; q < kLduNormBlocks; ++q) sum += h[q];
-    const double x_ref = sum / static_cast<double>(m.n);
-    k_norms<<<kLduNormBlocks, kNormThreads, 0, st>>>(m.n, m.nf, m.rp, m.ci, m.src, diag, upper, lower, b, x, x_ref,
-                                                     part);
-    CFDB_CUDA(cudaGetLastError());
-    CFDB_CUDA(cudaMemcpyAsync(h.data(), part, sizeof(double) * 3 * kLduNormBlocks, cudaMemcpyDeviceToHost, st));
-    CFDB_CUDA(cudaStreamSynchronize(st));
-    for (int q = 0; q < kLduNormBlocks; ++q) {
-        out.res += h[3 * q];
-        out.norm += h[3 * q + 1];
-        out.r2 += h[3 * q + 2];
+LduNorms Engine::residual_norms() {
+    CFDB_CUDA(cudaSetDevice(device_));
+    if (n_sys_ != 1) fail(1, "residual_norms: single-system plans only");
+    const DevLevel& d = lv_[0];
+    if (norms_ == nullptr) {
+        norms_ = arena_.alloc<NormState>(1);
+        // a second set of partials and tickets: the norms are three sums
+        const size_t groups = static_cast<size_t>(ceil_div(d.n_tiles, kGroupTiles)) + 1;
+        red2_ = red_;
+        red2_.partials = arena_.alloc<double>(2 * static_cast<size_t>(std::max(d.n_tiles, 1)));
+        red2_.gpartials = arena_.alloc<double>(2 * groups);
+        int* cnt = arena_.alloc<int>(1 + groups);
+        CFDB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * (1 + groups), stream_));
+        red2_.counters = cnt;
+        red2_.gcounters = cnt + 1;
     }
-    return out;
+    const bool pdl = tuning_.pdl != 0;
+    const int n = n_of_[0];
+    launch_k(pdl, k_ldu_mean, d.n_tiles, kBlock, 0, stream_, d.tiles, n, x_, red_, norms_);
+    if (row_width(d.a) <= 5.25)
+        launch_k(pdl, k_ldu_norms<5>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, n, b_, x_, red_, red2_, norms_);
+    else
+        launch_k(pdl, k_ldu_norms<7>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, n, b_, x_, red_, red2_, norms_);
+    launches_ += 2;
+    NormState* h = static_cast<NormState*>(h_state_.get(sizeof(NormState)));
+    CFDB_CUDA(cudaMemcpyAsync(h, norms_, sizeof(NormState), cudaMemcpyDeviceToHost, stream_));
+    CFDB_CUDA(cudaStreamSynchronize(stream_));
+    return LduNorms{h->res, h->norm, h->r2};
 }
 
 } // namespace cfdb
