@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <type_traits>
 
 namespace cfdb {
 
@@ -158,15 +159,53 @@ __global__ void k_ldu_values(int n, int nf, const int* __restrict__ dpos, const 
     }
 }
 
+// Row scans take G lanes per row (1, 8 or 32 by the average row length, with_lanes): one thread walks
+// a fine-level row of a few entries, but the rows of the coarse levels hold 100 to 400, and a thread
+// each left 3 to 37 CTAs serialising their loads (96 to 228 us a scan on levels of 9K and 700 rows).
+template <int G> struct RowLanes {
+    int i, lane;
+    unsigned mask; // the row's lanes in the warp
+    __device__ __forceinline__ RowLanes() {
+        const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+        i = static_cast<int>(t / G);
+        lane = static_cast<int>(threadIdx.x) & (G - 1);
+        const int w0 = static_cast<int>(threadIdx.x) & 31 & ~(G - 1);
+        mask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << w0;
+    }
+    // this lane's position among the row's lanes with pred, and their number
+    __device__ __forceinline__ int rank(bool pred, int& total) const {
+        if constexpr (G == 1) {
+            total = pred ? 1 : 0;
+            return 0;
+        } else {
+            const unsigned bal = __ballot_sync(mask, pred) & mask;
+            total = __popc(bal);
+            return __popc(bal & ((1u << (threadIdx.x & 31)) - 1u));
+        }
+    }
+    template <class T> __device__ __forceinline__ T sum(T v) const {
+        if constexpr (G > 1)
+            for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+        return v;
+    }
+    __device__ __forceinline__ int max(int v) const {
+        if constexpr (G > 1)
+            for (int o = G / 2; o > 0; o >>= 1) v = ::max(v, __shfl_xor_sync(mask, v, o));
+        return v;
+    }
+};
+
 // last diagonal entry of each row (any value), 0 if none
+template <int G>
 __global__ void k_last_diag(int n, const int* __restrict__ rp, const int* __restrict__ ci,
                             const double* __restrict__ va, double* d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double v = 0.0;
-    for (int k = rp[i]; k < rp[i + 1]; ++k)
-        if (ci[k] == i) v = va[k];
-    d[i] = v;
+    const RowLanes<G> r;
+    if (r.i >= n) return;
+    int at = -1;
+    for (int k = rp[r.i] + r.lane; k < rp[r.i + 1]; k += G)
+        if (ci[k] == r.i) at = k;
+    at = r.max(at);
+    if (r.lane == 0) d[r.i] = at >= 0 ? va[at] : 0.0;
 }
 
 __device__ __forceinline__ bool strong_entry(int i, int j, double v, double di, const double* d, double theta) {
@@ -174,26 +213,38 @@ __device__ __forceinline__ bool strong_entry(int i, int j, double v, double di, 
 }
 
 // FILL = false: number of strong entries per row; true: their columns and |a_ij|
-template <bool FILL>
+template <bool FILL, int G>
 __global__ void k_strong(int n, const int* __restrict__ rp, const int* __restrict__ ci,
                          const double* __restrict__ va, const double* __restrict__ d, double theta, int* cnt,
                          const int* __restrict__ srp, int* sci, double* sav) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const RowLanes<G> r;
+    const int i = r.i;
     if (i >= n) return;
     const double di = d[i];
     int c = 0;
     const int o = FILL ? srp[i] : 0;
-    for (int k = rp[i]; k < rp[i + 1]; ++k) {
-        const int j = ci[k];
-        if (strong_entry(i, j, va[k], di, d, theta)) {
-            if (FILL) {
-                sci[o + c] = j;
-                sav[o + c] = fabs(va[k]);
+    const int e = rp[i + 1];
+    for (int k0 = rp[i]; k0 < e; k0 += G) {
+        const int k = k0 + r.lane;
+        const int j = k < e ? ci[k] : i;
+        const double v = k < e ? va[k] : 0.0;
+        const bool strong = k < e && strong_entry(i, j, v, di, d, theta);
+        if (FILL) {
+            int total = 0;
+            const int at = r.rank(strong, total);
+            if (strong) {
+                sci[o + c + at] = j;
+                sav[o + c + at] = fabs(v);
             }
-            ++c;
+            c += total;
+        } else {
+            c += strong ? 1 : 0;
         }
     }
-    if (!FILL) cnt[i] = c;
+    if (!FILL) {
+        c = r.sum(c);
+        if (r.lane == 0) cnt[i] = c;
+    }
 }
 
 // rank of each strong entry within its row by (|a| descending, position ascending); rows have
@@ -233,6 +284,12 @@ __global__ void k_max_degree(int n, const int* __restrict__ srp, int* out) {
 // Decisions happen only near the smallest undecided row `lo` (a seed needs every earlier
 // conflict decided), so a sweep visits the window [lo, lo + kSeedWindow) and records the next
 // lo; sweeps run in batches on the device, the host reading lo once per batch.
+// What bounds this is the chain of decisions (a few hundred links on a mesh of 50 to 100 cells a
+// side): each row's earlier conflicts are listed once beforehand, a row steps through its list with
+// several states loaded at once, and a waiting row looks again up to kSeedPolls times within a sweep,
+// so that a link costs about one L2 load. Walking the graph and its transpose for every look cost 20
+// to 30 dependent loads a link: 288 sweeps of one look, 3.7 ms, on the 750K-cell tet box. The looks are
+// bounded and nothing depends on how far they get: a row still waiting is left to the next sweep.
 enum : int { kUndecided = 0, kSeed = 1, kNotSeed = 2 };
 
 __global__ void k_seed_init(int n, const int* __restrict__ srp, int* state) {
@@ -240,56 +297,90 @@ __global__ void k_seed_init(int n, const int* __restrict__ srp, int* state) {
     if (i < n) state[i] = srp[i + 1] > srp[i] ? kUndecided : kNotSeed;
 }
 
-constexpr int kSeedWindow = 1 << 18;
-constexpr int kSeedBatch = 32;  // sweeps per host check
+constexpr int kSeedWindow = 1 << 20; // 2^18: 12.3 against 10.6 ms of aggregation on the 5.1M-cell tet box
+constexpr int kSeedBatch = 4;   // sweeps per host check
+constexpr int kSeedPolls = 128; // looks of a row per sweep
+constexpr int kSeedLook = 8;    // conflicts looked at together
+
+// The earlier conflicts of every row (FILL = false: their number): for each j in N[i], the rows s < i
+// with j in N[s]. A row may be listed more than once.
+template <bool FILL>
+__global__ void k_conflicts(int n, const int* __restrict__ srp, const int* __restrict__ sci,
+                            const int* __restrict__ trp, const int* __restrict__ tci, int* cnt,
+                            const int* __restrict__ crp, int* cci) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int c = FILL ? crp[i] : 0;
+    const int k0 = srp[i], k1 = srp[i + 1];
+    if (k1 > k0) { // a row without strong connections is no seed: it needs none
+        for (int k = k0 - 1; k < k1; ++k) {
+            const int j = k < k0 ? i : sci[k];
+            if (j < i) { // s = j itself
+                if (FILL) cci[c] = j;
+                ++c;
+            }
+            for (int q = trp[j]; q < trp[j + 1]; ++q) {
+                const int s = tci[q];
+                if (s >= i) break;
+                if (FILL) cci[c] = s;
+                ++c;
+            }
+        }
+    }
+    if (!FILL) cnt[i] = c;
+}
 
 // One sweep over the rows [lo, lo + kSeedWindow), lo = *lo_in (every row below it is decided);
 // *lo_out receives the smallest row still undecided, or lo + kSeedWindow when the window
-// settled (*lo_out preset to INT_MAX). trp / tci: the transpose of S, rows ascending. For each
-// j in N[i] the earlier rows s with j in N[s] are scanned in ascending order up to the first one
-// not known to be a non-seed: a seed decides row i at once; an undecided one makes row i wait,
-// and the scan moves on to the next j, where a seed may still decide it.
-__global__ void k_seed_sweep(int n, const int* __restrict__ lo_in, int* lo_out, const int* __restrict__ srp,
-                             const int* __restrict__ sci, const int* __restrict__ trp, const int* __restrict__ tci,
-                             int* state_) {
+// settled (*lo_out preset to INT_MAX). crp / cci: the earlier conflicts; at[i]: how many of row i's
+// are known not to be seeds (kept between sweeps). The loop is flat, one look per turn, so that the
+// lanes of a warp that can decide are never held back by waiting ones.
+__global__ void k_seed_sweep(int n, const int* __restrict__ lo_in, int* lo_out, const int* __restrict__ crp,
+                             const int* __restrict__ cci, int* at, int* state_) {
     const int lo = *lo_in;
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicMin(lo_out, static_cast<int>(min(static_cast<long long>(lo) + kSeedWindow, static_cast<long long>(n))));
     const long long ii = static_cast<long long>(lo) + static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (ii >= n) return;
-    const int i = static_cast<int>(ii);
     volatile int* state = state_;
-    if (state[i] != kUndecided) return;
-    bool waiting = false;
-    for (int k = srp[i] - 1; k < srp[i + 1]; ++k) {
-        const int j = k < srp[i] ? i : sci[k];
-        if (j < i) {  // s = j itself
-            const int v = state[j];
-            if (v == kSeed) {
-                state[i] = kNotSeed;
-                return;
+    const int i = ii < n ? static_cast<int>(ii) : 0;
+    bool open = ii < n && state[i] == kUndecided;
+    int pos = 0, end = 0;
+    bool blocked = false; // c[0] was undecided at the last look
+    int c[kSeedLook];
+    if (open) {
+        end = crp[i + 1];
+        pos = crp[i] + at[i];
+    }
+    for (int turn = 0; turn < kSeedPolls; ++turn) {
+        if (!__any_sync(0xffffffffu, open)) break;
+        if (!open || (blocked && state[c[0]] == kUndecided)) continue;
+        // the next conflicts in order, from the first one not yet passed
+#pragma unroll
+        for (int u = 0; u < kSeedLook; ++u) c[u] = pos + u < end ? cci[pos + u] : -1;
+        int v[kSeedLook];
+#pragma unroll
+        for (int u = 0; u < kSeedLook; ++u) v[u] = c[u] >= 0 ? state[c[u]] : kNotSeed;
+        bool seed = false, clear = true;
+        int passed = 0;
+#pragma unroll
+        for (int u = 0; u < kSeedLook; ++u) {
+            seed = seed || v[u] == kSeed;
+            if (clear && v[u] != kNotSeed) {
+                clear = false;
+                c[0] = c[u]; // waits for this one
             }
-            if (v == kUndecided) {
-                waiting = true;
-                continue;
-            }
+            passed += clear && c[u] >= 0 ? 1 : 0;
         }
-        for (int q = trp[j]; q < trp[j + 1]; ++q) {
-            const int s = tci[q];
-            if (s >= i) break;
-            const int v = state[s];
-            if (v == kSeed) {
-                state[i] = kNotSeed;
-                return;
-            }
-            if (v == kUndecided) {
-                waiting = true;
-                break;
-            }
+        pos += passed;
+        blocked = !clear;
+        if (seed || pos >= end) {
+            state[i] = seed ? kNotSeed : kSeed;
+            open = false;
         }
     }
-    if (waiting) atomicMin(lo_out, i);
-    else state[i] = kSeed;
+    if (open) at[i] = pos - crp[i];
+    const int left = __reduce_min_sync(0xffffffffu, open ? i : INT_MAX);
+    if (left != INT_MAX && (threadIdx.x & 31) == 0) atomicMin(lo_out, left);
 }
 
 __global__ void k_seed_flags(int n, const int* __restrict__ state, int* flag) {
@@ -360,18 +451,29 @@ __global__ void k_pass3(int n_left, const int* __restrict__ list, const int* __r
     *n_agg = a;
 }
 
-// inv = 1/d (0 where d == 0); rho = max_i |inv_i| sum_j |a_ij| (bits of a non-negative double)
-__global__ void k_inv_rho(int n, const int* __restrict__ rp, const double* __restrict__ va,
+// inv = 1/d (0 where d == 0); rho = max_i |inv_i| sum_j |a_ij| (bits of a non-negative double: one
+// atomic per block; one per row took 499 us on 750K rows)
+__global__ void __launch_bounds__(kThreads) k_inv_rho(int n, const int* __restrict__ rp, const double* __restrict__ va,
                           const double* __restrict__ d, double* inv, unsigned long long* rho_bits) {
+    __shared__ unsigned long long sh[kThreads / 32];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double di = d[i];
-    const double iv = di != 0.0 ? __ddiv_rn(1.0, di) : 0.0;
-    inv[i] = iv;
-    double row = 0.0;
-    for (int k = rp[i]; k < rp[i + 1]; ++k) row = __dadd_rn(row, fabs(va[k]));
-    const double v = __dmul_rn(row, fabs(iv));
-    if (v > 0.0) atomicMax(rho_bits, static_cast<unsigned long long>(__double_as_longlong(v)));
+    unsigned long long bits = 0;
+    if (i < n) {
+        const double di = d[i];
+        const double iv = di != 0.0 ? __ddiv_rn(1.0, di) : 0.0;
+        inv[i] = iv;
+        double row = 0.0;
+        for (int k = rp[i]; k < rp[i + 1]; ++k) row = __dadd_rn(row, fabs(va[k]));
+        const double v = __dmul_rn(row, fabs(iv));
+        if (v > 0.0) bits = static_cast<unsigned long long>(__double_as_longlong(v));
+    }
+    for (int o = 16; o > 0; o >>= 1) bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, o));
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = bits;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kThreads / 32; ++w) bits = max(bits, sh[w]);
+        if (bits != 0) atomicMax(rho_bits, bits);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -557,9 +659,11 @@ __global__ void __launch_bounds__(G* PER) k_gemm_rows(GemmArgs g) {
             const int total = __shfl_sync(full, inc, 31);
             const int exc = inc - len;
             bool stop = false;
-            for (int f0 = 0; f0 < total && !stop; f0 += 32) {
+            // a chunk's columns and factors are loaded while the chunk before it is added
+            int j_next = 0;
+            double a_next = 0.0, b_next = 0.0;
+            auto fetch = [&](int f0) {
                 const int f = f0 + lane;
-                const bool active = f < total;
                 int src = 0; // first lane whose inclusive prefix exceeds f
                 for (int step = 16; step > 0; step >>= 1) {
                     const int v = __shfl_sync(full, inc, src + step - 1);
@@ -567,10 +671,19 @@ __global__ void __launch_bounds__(G* PER) k_gemm_rows(GemmArgs g) {
                 }
                 const int off = f - __shfl_sync(full, exc, src);
                 const int kb = __shfl_sync(full, bstart, src) + off;
-                const double avs = __shfl_sync(full, av, src);
-                const int j = active ? (g.brp != nullptr ? g.bci[kb] : g.tent[kb]) : -1 - lane;
+                a_next = __shfl_sync(full, av, src);
+                const bool in = f < total;
+                j_next = in ? (g.brp != nullptr ? g.bci[kb] : g.tent[kb]) : -1 - lane;
+                if constexpr (NUMERIC) b_next = in && g.brp != nullptr ? g.bva[kb] : 1.0;
+            };
+            if (total > 0) fetch(0);
+            for (int f0 = 0; f0 < total && !stop; f0 += 32) {
+                const bool active = f0 + lane < total;
+                const int j = j_next;
+                const double avs = a_next, bv = b_next;
+                if (f0 + 32 < total) fetch(f0 + 32);
                 if constexpr (NUMERIC) {
-                    sv[lane] = active ? __dmul_rn(avs, g.brp != nullptr ? g.bva[kb] : 1.0) : 0.0;
+                    sv[lane] = active ? __dmul_rn(avs, bv) : 0.0;
                     const unsigned same = __match_any_sync(full, j);
                     __syncwarp();
                     if (active && lane == __ffs(same) - 1) {
@@ -604,15 +717,23 @@ __global__ void __launch_bounds__(G* PER) k_gemm_rows(GemmArgs g) {
             if (stop) break; // uniform within the warp
         }
     } else {
-        for (int ka = a0; ka < a1; ++ka) {
+        // the next k's row of B is located while the current one is added
+        int b0_next = 0, b1_next = 0;
+        double av_next = 0.0;
+        auto locate = [&](int ka) {
             const int k = g.aci[ka];
-            double av = 0.0;
+            if constexpr (NUMERIC) av_next = g.ava[ka];
+            b0_next = g.brp != nullptr ? g.brp[k] : k;
+            b1_next = g.brp != nullptr ? g.brp[k + 1] : k + 1;
+        };
+        if (a0 < a1) locate(a0);
+        for (int ka = a0; ka < a1; ++ka) {
+            const int b0 = b0_next, b1 = b1_next;
+            double av = av_next;
             if constexpr (NUMERIC) {
-                av = g.ava[ka];
                 if (g.ascale != nullptr) av = __dmul_rn(g.ascale[i], av);
             }
-            const int b0 = g.brp != nullptr ? g.brp[k] : k;
-            const int b1 = g.brp != nullptr ? g.brp[k + 1] : k + 1;
+            if (ka + 1 < a1) locate(ka + 1);
             for (int kb = b0 + t; kb < b1; kb += G) {
                 const int j = g.brp != nullptr ? g.bci[kb] : g.tent[kb];
                 bool fresh = false;
@@ -672,16 +793,18 @@ __global__ void __launch_bounds__(G* PER) k_gemm_rows(GemmArgs g) {
 }
 
 // upper bound of the distinct columns of row i of A B: min(sum_k |B(k,:)|, n_cols)
+template <int G>
 __global__ void k_gemm_bound(int n, const int* __restrict__ arp, const int* __restrict__ aci,
                              const int* __restrict__ brp, int n_cols, int* ub) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const RowLanes<G> r;
+    if (r.i >= n) return;
     long long u = 0;
-    for (int ka = arp[i]; ka < arp[i + 1]; ++ka) {
+    for (int ka = arp[r.i] + r.lane; ka < arp[r.i + 1]; ka += G) {
         const int k = aci[ka];
         u += brp != nullptr ? brp[k + 1] - brp[k] : 1;
     }
-    ub[i] = static_cast<int>(u < n_cols ? u : n_cols);
+    u = r.sum(u);
+    if (r.lane == 0) ub[r.i] = static_cast<int>(u < n_cols ? u : n_cols);
 }
 
 // Table-size classes of a row (distinct columns, or entries of a row to sort), smallest first:
@@ -794,6 +917,21 @@ __global__ void __launch_bounds__(G* PER) k_seg_sort(const int* __restrict__ row
     }
     const int r0 = rp[i], len = rp[i + 1] - r0;
     if (len > cap) return; // classified by length: cannot happen
+    if constexpr (G == 32) {
+        // up to 32 entries: every lane counts the keys below its own and stores its entry there
+        // (bitonic passes through shared memory took 226 us for 750K rows of 4 entries)
+        if (len <= 32) {
+            const int key = t < len ? ci[r0 + t] : kEmpty;
+            const double v = t < len ? va[r0 + t] : 0.0;
+            int at = 0;
+            for (int q = 0; q < len; ++q) at += __shfl_sync(0xffffffffu, key, q) < key ? 1 : 0;
+            if (t < len) {
+                ci[r0 + at] = key;
+                va[r0 + at] = v;
+            }
+            return;
+        }
+    }
     int p2 = 1;
     while (p2 < len) p2 <<= 1;
     for (int s = t; s < p2; s += G) {
@@ -808,25 +946,34 @@ __global__ void __launch_bounds__(G* PER) k_seg_sort(const int* __restrict__ row
     }
 }
 
+template <int G>
 __global__ void k_nz_count(int n, const int* __restrict__ rp, const double* __restrict__ va, int* cnt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const RowLanes<G> r;
+    if (r.i >= n) return;
     int c = 0;
-    for (int k = rp[i]; k < rp[i + 1]; ++k) c += va[k] != 0.0;
-    cnt[i] = c;
+    for (int k = rp[r.i] + r.lane; k < rp[r.i + 1]; k += G) c += va[k] != 0.0;
+    c = r.sum(c);
+    if (r.lane == 0) cnt[r.i] = c;
 }
 
+template <int G>
 __global__ void k_nz_compact(int n, const int* __restrict__ rp, const int* __restrict__ ci, const double* __restrict__ va,
                              const int* __restrict__ nrp, int* nci, double* nva) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int o = nrp[i];
-    for (int k = rp[i]; k < rp[i + 1]; ++k) {
-        if (va[k] != 0.0) {
-            nci[o] = ci[k];
-            nva[o] = va[k];
-            ++o;
+    const RowLanes<G> r;
+    if (r.i >= n) return;
+    int o = nrp[r.i];
+    const int e = rp[r.i + 1];
+    for (int k0 = rp[r.i]; k0 < e; k0 += G) {
+        const int k = k0 + r.lane;
+        const int j = k < e ? ci[k] : 0;
+        const double v = k < e ? va[k] : 0.0;
+        int total = 0;
+        const int at = r.rank(v != 0.0, total);
+        if (v != 0.0) {
+            nci[o + at] = j;
+            nva[o + at] = v;
         }
+        o += total;
     }
 }
 
@@ -857,6 +1004,14 @@ template <class T> void to_host(std::vector<T>& h, const T* d, size_t n, cudaStr
 }
 
 void sync(cudaStream_t st) { CFDB_CUDA(cudaStreamSynchronize(st)); }
+
+// fn with the lanes per row of a scan over n rows with nnz entries, and the grid for them.
+template <class Fn> void with_lanes(int n, long long nnz, Fn&& fn) {
+    const double avg = n > 0 ? static_cast<double>(nnz) / n : 0.0;
+    if (avg <= 8.0) fn(std::integral_constant<int, 1>{}, grid_for(n));
+    else if (avg <= 32.0) fn(std::integral_constant<int, 8>{}, grid_for(8LL * n));
+    else fn(std::integral_constant<int, 32>{}, grid_for(32LL * n));
+}
 
 // out[0..n] = exclusive scan of in[0..n), out[n] = total; returns the total.
 long long scan(Ctx& cx, const int* in, int n, int* out) {
@@ -937,6 +1092,8 @@ template <class K> void set_smem(K kernel, size_t bytes) {
     }
 }
 
+constexpr int kCtaRows = 148 * 8;
+
 // One Gustavson kernel launch over the rows of a list, with the table class `cls` (0..4).
 template <bool NUMERIC> void gemm_launch(Ctx& cx, GemmArgs g, int cls, const int* rows, int n_list) {
     if (n_list <= 0) return;
@@ -945,6 +1102,9 @@ template <bool NUMERIC> void gemm_launch(Ctx& cx, GemmArgs g, int cls, const int
     const size_t b = NUMERIC ? 12 : 4;      // bytes per slot
     const size_t chunk = NUMERIC ? 32 * 8 : 0; // warp groups: one chunk of contributions
     cudaStream_t st = cx.st;
+    // few rows of many entries: a CTA per row, whose threads take a whole row of B at once, instead of a
+    // warp walking its contributions 32 at a time (556 rows of a 3.7K-row level: 752 us)
+    if (cls == 2 && n_list <= kCtaRows) cls = 3;
     switch (cls) {
     case 0:
         k_gemm_rows<NUMERIC, 32, 64, 8><<<(n_list + 7) / 8, 256, 8 * (64 * b + chunk), st>>>(g);
@@ -987,7 +1147,10 @@ DevCsr spgemm(Ctx& cx, const DevCsr& a, const double* ascale, const DevCsr* b, c
     // there; the others start in the 512-slot warp tables and move to larger tables when they
     // fill up (the bound is loose: most such rows have far fewer distinct columns)
     int* ub = cx.mem->alloc<int>(std::max(n, 1));
-    if (n > 0) k_gemm_bound<<<grid_for(n), kThreads, 0, st>>>(n, a.rp, a.ci, g.brp, n_cols, ub);
+    if (n > 0)
+        with_lanes(n, a.nnz, [&](auto G, int grid) {
+            k_gemm_bound<decltype(G)::value><<<grid, kThreads, 0, st>>>(n, a.rp, a.ci, g.brp, n_cols, ub);
+        });
     int* cnt = cx.mem->alloc<int>(static_cast<size_t>(n) + 1);
     g.cnt = cnt;
     const Classes sc = classify(cx, n, ub, kFill);
@@ -1128,13 +1291,18 @@ DevCsr prune_zeros(Ctx& cx, const DevCsr& a) {
     o.n_rows = a.n_rows;
     o.n_cols = a.n_cols;
     int* cnt = cx.mem->alloc<int>(static_cast<size_t>(a.n_rows) + 1);
-    if (a.n_rows > 0) k_nz_count<<<grid_for(a.n_rows), kThreads, 0, st>>>(a.n_rows, a.rp, a.va, cnt);
+    if (a.n_rows > 0)
+        with_lanes(a.n_rows, a.nnz, [&](auto G, int grid) {
+            k_nz_count<decltype(G)::value><<<grid, kThreads, 0, st>>>(a.n_rows, a.rp, a.va, cnt);
+        });
     o.rp = cx.out<int>(static_cast<size_t>(a.n_rows) + 1);
     o.nnz = checked_nnz(scan(cx, cnt, a.n_rows, o.rp), "a coarse operator");
     o.ci = cx.out<int>(static_cast<size_t>(o.nnz) + 4);
     o.va = cx.out<double>(static_cast<size_t>(o.nnz) + 4);
     if (a.n_rows > 0)
-        k_nz_compact<<<grid_for(a.n_rows), kThreads, 0, st>>>(a.n_rows, a.rp, a.ci, a.va, o.rp, o.ci, o.va);
+        with_lanes(a.n_rows, a.nnz, [&](auto G, int grid) {
+            k_nz_compact<decltype(G)::value><<<grid, kThreads, 0, st>>>(a.n_rows, a.rp, a.ci, a.va, o.rp, o.ci, o.va);
+        });
     CFDB_CUDA(cudaGetLastError());
     return o;
 }
@@ -1142,19 +1310,18 @@ DevCsr prune_zeros(Ctx& cx, const DevCsr& a) {
 // Rows left by pass 2 that pass 3 runs on the device (one thread); more go to the host.
 constexpr int kPass3Device = 1024;
 
-// Levels aggregated on the device: large and sparse ones (the fine level of a mesh). Each
-// pass-1 sweep costs microseconds and more with every strong entry per row, while the host's
-// sequential pass costs nanoseconds per strong entry plus the strength graph's read-back.
-// Measured on the jittered 6-tet box of 5.1M cells: the fine level (3.9 strong entries per row)
-// 14 ms on the device (930 sweeps) against 21.5 ms on the host plus 3 ms of read-back; the first
-// coarse level (861K rows, 8.7 per row) 16 ms against 11 ms.
-bool device_aggregation(int n, long long ns) { return n >= (1 << 18) && ns <= 6LL * n; }
+// Levels aggregated on the device: all but the small and the dense ones (the conflict lists grow with
+// the square of the strong entries per row, while the host's sequential pass costs nanoseconds per
+// strong entry plus the strength graph's read-back). Measured, aggregation phase of all levels with
+// the host from 262K rows or 6 strong entries per row down, against this line: tet 95^3x6 22.1 / 14.9
+// ms (its second level: 861K rows of 8.7), tet 50^3x6 4.4 / 3.6, tet 30^3x6 1.9 / 1.3, graded 64^3 2.6 / 2.1.
+bool device_aggregation(int n, long long ns) { return n >= 4096 && ns <= 20LL * n; }
 
 // The aggregation on the device from the strength graph (srp, sci, sav = |a_ij|): passes 1 and
 // 2 in parallel, pass 3 by one thread when at most kPass3Device rows are left for it. agg
 // receives every row's aggregate. Returns the number of aggregates, or -1 when more rows are
-// left for pass 3 (isolated rows, or rows none of whose strong neighbours pass 1 aggregated):
-// the caller then aggregates on the host.
+// left for pass 3 (isolated rows, or rows none of whose strong neighbours pass 1 aggregated), or the
+// conflict lists pass 2^31 entries: the caller then aggregates on the host.
 int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, int* agg) {
     cudaStream_t st = cx.st;
     Ctx tx = cx;
@@ -1169,6 +1336,15 @@ int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, in
     int* state = cx.mem->alloc<int>(n);
     int* counter = cx.d_counts + kClasses; // the spare counter
     k_seed_init<<<grid_for(n), kThreads, 0, st>>>(n, srp, state);
+    int* ccnt = cx.mem->alloc<int>(static_cast<size_t>(n) + 1);
+    int* crp = cx.mem->alloc<int>(static_cast<size_t>(n) + 1);
+    k_conflicts<false><<<grid_for(n), kThreads, 0, st>>>(n, srp, sci, t.rp, t.ci, ccnt, nullptr, nullptr);
+    const long long n_conf = scan(cx, ccnt, n, crp);
+    if (n_conf > INT_MAX) return -1;
+    int* cci = cx.mem->alloc<int>(static_cast<size_t>(n_conf));
+    k_conflicts<true><<<grid_for(n), kThreads, 0, st>>>(n, srp, sci, t.rp, t.ci, nullptr, crp, cci);
+    int* at = ccnt; // conflicts passed so far
+    CFDB_CUDA(cudaMemsetAsync(at, 0, sizeof(int) * static_cast<size_t>(n), st));
     // lo of each sweep of a batch; lo[0] = 0, then the last lo of the previous batch
     int* lo = cx.mem->alloc<int>(kSeedBatch + 1);
     CFDB_CUDA(cudaMemsetAsync(lo, 0, sizeof(int), st));
@@ -1178,7 +1354,7 @@ int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, in
         if (sweeps > n + kSeedBatch) fail(kErrInternal, "device aggregation did not settle");
         CFDB_CUDA(cudaMemsetAsync(lo + 1, 0x7f, sizeof(int) * kSeedBatch, st));
         for (int b = 0; b < kSeedBatch; ++b)
-            k_seed_sweep<<<grid, kThreads, 0, st>>>(n, lo + b, lo + b + 1, srp, sci, t.rp, t.ci, state);
+            k_seed_sweep<<<grid, kThreads, 0, st>>>(n, lo + b, lo + b + 1, crp, cci, at, state);
         CFDB_CUDA(cudaGetLastError());
         sweeps += kSeedBatch;
         int last = 0;
@@ -1266,7 +1442,9 @@ void amg_setup_device(const DevCsr& a0, const AmgSettings& s, cudaStream_t st, D
     for (int l = 0; l < s.max_levels; ++l) {
         const int nl = cur.n_rows;
         double* d = h.mem.alloc<double>(nl);
-        k_last_diag<<<grid_for(nl), kThreads, 0, st>>>(nl, cur.rp, cur.ci, cur.va, d);
+        with_lanes(nl, cur.nnz, [&](auto G, int grid) {
+            k_last_diag<decltype(G)::value><<<grid, kThreads, 0, st>>>(nl, cur.rp, cur.ci, cur.va, d);
+        });
         const bool last = nl <= s.coarse_size || l + 1 == s.max_levels;
         if (last) {
             h.a.push_back(cur);
@@ -1274,14 +1452,18 @@ void amg_setup_device(const DevCsr& a0, const AmgSettings& s, cudaStream_t st, D
         }
         // strength graph
         int* scnt = h.mem.alloc<int>(static_cast<size_t>(nl) + 1);
-        k_strong<false><<<grid_for(nl), kThreads, 0, st>>>(nl, cur.rp, cur.ci, cur.va, d, s.theta, scnt, nullptr,
-                                                           nullptr, nullptr);
+        with_lanes(nl, cur.nnz, [&](auto G, int grid) {
+            k_strong<false, decltype(G)::value><<<grid, kThreads, 0, st>>>(nl, cur.rp, cur.ci, cur.va, d, s.theta, scnt,
+                                                                           nullptr, nullptr, nullptr);
+        });
         int* srp = h.mem.alloc<int>(static_cast<size_t>(nl) + 1);
         const int ns = checked_nnz(scan(cx, scnt, nl, srp), "the strength graph");
         int* sci = h.mem.alloc<int>(ns);
         double* sav = h.mem.alloc<double>(ns);
-        k_strong<true><<<grid_for(nl), kThreads, 0, st>>>(nl, cur.rp, cur.ci, cur.va, d, s.theta, nullptr, srp, sci,
-                                                          sav);
+        with_lanes(nl, cur.nnz, [&](auto G, int grid) {
+            k_strong<true, decltype(G)::value><<<grid, kThreads, 0, st>>>(nl, cur.rp, cur.ci, cur.va, d, s.theta, nullptr,
+                                                                          srp, sci, sav);
+        });
         CFDB_CUDA(cudaGetLastError());
         phase("strength");
         // aggregation: passes 1 and 2 on the device; when rows are left for pass 3 the host runs
@@ -1481,17 +1663,21 @@ __global__ void k_sell_fill(int n, int n_sl, const int* __restrict__ perm, const
     }
 }
 
+template <int G>
 __global__ void k_weighted_inv_diag(int n, int n_pad, const int* __restrict__ rp, const int* __restrict__ ci,
                                     const double* __restrict__ va, double weight, double* wd64, float* wd32) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const RowLanes<G> r;
+    const int i = r.i;
     if (i >= n_pad) return;
     double w = weight;
     if (i < n) {
-        double dinv = 1.0;
-        for (int k = rp[i]; k < rp[i + 1]; ++k)
-            if (ci[k] == i && va[k] != 0.0) dinv = __ddiv_rn(1.0, va[k]);
-        w = __dmul_rn(weight, dinv);
+        int at = -1; // the last nonzero diagonal entry
+        for (int k = rp[i] + r.lane; k < rp[i + 1]; k += G)
+            if (ci[k] == i && va[k] != 0.0) at = k;
+        at = r.max(at);
+        w = __dmul_rn(weight, at >= 0 ? __ddiv_rn(1.0, va[at]) : 1.0);
     }
+    if (r.lane != 0) return;
     if (wd64 != nullptr) wd64[i] = w;
     if (wd32 != nullptr) wd32[i] = __double2float_rn(w);
 }
@@ -1570,7 +1756,10 @@ void sell_fill(const DevCsr& m, int n_pad, const int* perm, const int* slice, in
 
 void weighted_inverse_diagonal(const DevCsr& m, int n_pad, double weight, double* wd64, float* wd32, cudaStream_t st) {
     if (n_pad > 0)
-        k_weighted_inv_diag<<<grid_for(n_pad), kThreads, 0, st>>>(m.n_rows, n_pad, m.rp, m.ci, m.va, weight, wd64, wd32);
+        with_lanes(n_pad, m.nnz, [&](auto G, int grid) {
+            k_weighted_inv_diag<decltype(G)::value><<<grid, kThreads, 0, st>>>(m.n_rows, n_pad, m.rp, m.ci, m.va, weight,
+                                                                               wd64, wd32);
+        });
     CFDB_CUDA(cudaGetLastError());
 }
 
