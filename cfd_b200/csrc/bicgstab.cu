@@ -52,6 +52,7 @@ static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>))
     int* n_active) {
     pdl_launch();
     const TileCtx c = tile_of(tiles);
+    reduce_begin(c.tile, c.s, red);
     Visit<V, double> vis;
     vis.begin(a, c.r0, c.r1);
     pdl_wait();
@@ -65,7 +66,7 @@ static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>))
                 v[row] = 0.0;
                 rr = __dadd_rn(rr, __dmul_rn(ri, ri));
             });
-    if (reduce_system(rr, unused, c.tile, c.s, red) && threadIdx.x == 0) {
+    if (reduce_system(rr, unused, c.tile, red) && threadIdx.x == 0) {
         BcgState& s = *st;
         s.res = sqrt(rr);
         if (s.res <= s.tol) {
@@ -121,6 +122,7 @@ static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>))
     double* __restrict__ out, Reduce red, int* n_active) {
     pdl_launch();
     const TileCtx c = tile_of(tiles);
+    reduce_begin(c.tile, c.s, red);
     Visit<V, double> vis;
     vis.begin(a, c.r0, c.r1);
     pdl_wait();
@@ -137,7 +139,7 @@ static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>))
                     d0 = __dadd_rn(d0, __dmul_rn(wi, q));
                 }
             });
-    if (reduce_system(d0, d1, c.tile, c.s, red) && threadIdx.x == 0) {
+    if (reduce_system(d0, d1, c.tile, red) && threadIdx.x == 0) {
         BcgState& s = *st;
         if (kSecond) {
             s.omega = d0 > 0.0 ? d1 / d0 : 0.0;
@@ -156,6 +158,7 @@ static __global__ void __launch_bounds__(kBlock) k_bcg_s(Tiles tiles, BcgState* 
                                                          double* __restrict__ sh, Reduce red) {
     pdl_launch();
     const TileCtx c = tile_of(tiles);
+    reduce_begin(c.tile, c.s, red);
     pdl_wait();
     if (!bcg_active(st)) return;
     const double alpha = st->alpha;
@@ -180,7 +183,7 @@ static __global__ void __launch_bounds__(kBlock) k_bcg_s(Tiles tiles, BcgState* 
             ss = __dadd_rn(ss, __dmul_rn(si, si));
         }
     }
-    if (reduce_system(ss, unused, c.tile, c.s, red) && threadIdx.x == 0) {
+    if (reduce_system(ss, unused, c.tile, red) && threadIdx.x == 0) {
         BcgState& q = *st;
         const double norm = sqrt(ss);
         q.half = norm <= q.tol ? 1 : 0;
@@ -198,6 +201,7 @@ static __global__ void __launch_bounds__(kBlock) k_bcg_xr(Tiles tiles, BcgState*
                                                           double* __restrict__ r, Reduce red, int* n_active) {
     pdl_launch();
     const TileCtx c = tile_of(tiles);
+    reduce_begin(c.tile, c.s, red);
     pdl_wait();
     if (!bcg_active(st)) return;
     const double alpha = st->alpha, omega = st->omega;
@@ -231,7 +235,7 @@ static __global__ void __launch_bounds__(kBlock) k_bcg_xr(Tiles tiles, BcgState*
             }
         }
     }
-    if (reduce_system(rr, rho, c.tile, c.s, red) && threadIdx.x == 0) {
+    if (reduce_system(rr, rho, c.tile, red) && threadIdx.x == 0) {
         BcgState& q = *st;
         if (half) {
             bcg_stop(q, q.it, 1, n_active);

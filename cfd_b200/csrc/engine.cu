@@ -841,10 +841,10 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
         const int n_groups = std::max(grp0[n_sys_], 1);
         red_.partials = arena_.alloc<double>(2 * static_cast<size_t>(std::max(lv_[0].n_tiles, 1)));
         red_.gpartials = arena_.alloc<double>(2 * static_cast<size_t>(n_groups));
-        int* cnt = arena_.alloc<int>(n_sys_ + n_groups);
-        CFDB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * (n_sys_ + n_groups), st));
+        int* cnt = arena_.alloc<int>(2 * n_groups);
+        CFDB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * 2 * n_groups, st));
         red_.counters = cnt;
-        red_.gcounters = cnt + n_sys_;
+        red_.gcounters = cnt + n_groups;
         red_.sys_tile0 = arena_.upload(sys_tile0, st);
         red_.grp0 = arena_.upload(grp0, st);
         seq_ = arena_.alloc<int>(1);

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(kBlock) k_ldu_mean(Tiles tiles, int n, const d
                                                      NormState* out) {
     pdl_launch();
     const TileCtx c = tile_of(tiles);
+    reduce_begin(c.tile, c.s, red);
     pdl_wait();
     double s = 0.0, unused = 0.0;
     for (int r0 = c.r0 + threadIdx.x; r0 < c.r1; r0 += 4 * kBlock) {
@@ -35,7 +36,7 @@ __global__ void __launch_bounds__(kBlock) k_ldu_mean(Tiles tiles, int n, const d
 #pragma unroll
         for (int u = 0; u < 4; ++u) s += v[u];
     }
-    if (reduce_system(s, unused, c.tile, c.s, red) && threadIdx.x == 0) out->x_ref = s / static_cast<double>(n);
+    if (reduce_system(s, unused, c.tile, red) && threadIdx.x == 0) out->x_ref = s / static_cast<double>(n);
 }
 
 // sum |b - Ax|, sum |Ax - rs x_ref| + |b - rs x_ref| (rs = row sum), sum (b - Ax)^2 over the n user
@@ -46,6 +47,7 @@ __global__ void __launch_bounds__(kBlock) k_ldu_norms(Sell<double> m, Tiles tile
                                                       NormState* out) {
     pdl_launch();
     const TileCtx c = tile_of(tiles);
+    reduce_begin(c.tile, c.s, red);
     pdl_wait();
     const double x_ref = *reinterpret_cast<volatile const double*>(&out->x_ref);
     double res = 0.0, norm = 0.0, r2 = 0.0, unused = 0.0;
@@ -72,11 +74,11 @@ __global__ void __launch_bounds__(kBlock) k_ldu_norms(Sell<double> m, Tiles tile
         norm += fabs(ax - ax_ref) + fabs(bi - ax_ref);
         r2 += __dmul_rn(ri, ri);
     }
-    if (reduce_system(res, norm, c.tile, c.s, red) && threadIdx.x == 0) {
+    if (reduce_system(res, norm, c.tile, red) && threadIdx.x == 0) {
         out->res = res;
         out->norm = norm;
     }
-    if (reduce_system(r2, unused, c.tile, c.s, red2) && threadIdx.x == 0) out->r2 = r2;
+    if (reduce_system(r2, unused, c.tile, red2) && threadIdx.x == 0) out->r2 = r2;
 }
 
 } // namespace
@@ -92,10 +94,10 @@ LduNorms Engine::residual_norms() {
         red2_ = red_;
         red2_.partials = arena_.alloc<double>(2 * static_cast<size_t>(std::max(d.n_tiles, 1)));
         red2_.gpartials = arena_.alloc<double>(2 * groups);
-        int* cnt = arena_.alloc<int>(1 + groups);
-        CFDB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * (1 + groups), stream_));
+        int* cnt = arena_.alloc<int>(2 * groups);
+        CFDB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * 2 * groups, stream_));
         red2_.counters = cnt;
-        red2_.gcounters = cnt + 1;
+        red2_.gcounters = cnt + groups;
     }
     const bool pdl = tuning_.pdl != 0;
     const int n = n_of_[0];
