@@ -1776,26 +1776,33 @@ std::vector<SolveResult> Engine::solve(Mode mode, const std::vector<SolveRequest
     // A system takes at most max_it iterations and the preconditioning that finds the limit passed.
     // In mixed precision the systems at the target are then checked in FP64 together; those that
     // fail iterate on (at least one iteration each, so there are at most max_it such rounds).
-    for (int round = 0; round <= max_it; ++round) {
-        iterate(row, max_it + 2);
-        if (mode == Mode::AmgMixed) launch_graph(row, kVerify);
-        CFDB_CUDA(cudaMemcpyAsync(hs, st_, st_bytes, cudaMemcpyDeviceToHost, stream_));
-        CFDB_CUDA(cudaStreamSynchronize(stream_));
-        if (words[1] != 0) fail_wait(words[1]);
-        if (mode != Mode::AmgMixed || words[0] <= 0) break;
-    }
-    // true residuals for reporting, where the check has not just computed them
-    bool missing = false;
-    for (int s = 0; s < n_sys_ && want_true; ++s) missing = missing || !(hs[s].converged && hs[s].true_res >= 0.0);
-    if (missing) {
+    auto true_residuals = [&] {
         const DevLevel& d = lv_[0];
         with_krylov_visit(krylov_visit(), [&](auto V) {
             launch_k(tuning_.pdl != 0, k_true_residual<decltype(V)::value>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, st_, b_, x_, red_);
         });
         ++launches_;
         CFDB_CUDA(cudaGetLastError());
+    };
+    auto read_states = [&] {
         CFDB_CUDA(cudaMemcpyAsync(hs, st_, st_bytes, cudaMemcpyDeviceToHost, stream_));
         CFDB_CUDA(cudaStreamSynchronize(stream_));
+    };
+    for (int round = 0; round <= max_it; ++round) {
+        iterate(row, max_it + 2);
+        if (mode == Mode::AmgMixed) launch_graph(row, kVerify);
+        else if (want_true) true_residuals();
+        read_states();
+        if (words[1] != 0) fail_wait(words[1]);
+        if (mode != Mode::AmgMixed || words[0] <= 0) break;
+    }
+    // mixed precision: true residuals for reporting, where the check has not computed the last one
+    bool missing = false;
+    for (int s = 0; s < n_sys_ && want_true && mode == Mode::AmgMixed; ++s)
+        missing = missing || !(hs[s].converged && hs[s].true_res >= 0.0);
+    if (missing) {
+        true_residuals();
+        read_states();
     }
     std::vector<SolveResult> out(n_sys_);
     for (int s = 0; s < n_sys_; ++s) {
