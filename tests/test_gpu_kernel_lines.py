@@ -1,0 +1,216 @@
+"""The device kernels at the lines where their work is split differently: row widths of the SELL
+and lane-group visits, tile counts of the reductions, row lengths of the setup's products and
+sorts. Each against the oracle or the host build; whole numbers and fixed-order sums bit for bit,
+reordered FP64 sums within their round-off bound."""
+import numpy as np
+import pytest
+
+import oracle as O
+from cfd_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(np.float64).eps
+
+
+def _banded(n, half, seed=3):
+    """Symmetric, diagonally dominant matrix with 2 half + 1 entries in the rows away from the ends."""
+    i = np.arange(n)
+    pairs = np.concatenate([np.stack([i[:n - k], i[k:]], 1) for k in range(1, half + 1)])
+    pairs = pairs[np.lexsort((pairs[:, 1], pairs[:, 0]))]
+    own, nei = pairs[:, 0].astype(np.int32), pairs[:, 1].astype(np.int32)
+    rng = np.random.default_rng(seed)
+    w = rng.uniform(0.5, 1.5, len(own))
+    diag = np.bincount(own, w, n) + np.bincount(nei, w, n) + 0.05
+    return own, nei, -w, -w.copy(), diag, rng.standard_normal(n)
+
+
+def _pressure(case):
+    up, lo, dg, dv = O.assemble(case.n, case.owner, case.neighbour, case.flux, case.gamma,
+                                case.delta, 0.0)
+    diag, src = case.finalize(up, lo, dg, dv)
+    return up, lo, diag, src
+
+
+def _csr(n, own, nei, diag, up, lo):
+    return O.ldu_to_csr(O.build_pattern(n, own, nei), diag, up, lo)
+
+
+@pytest.mark.parametrize("n", [33, 255, 257, 20001])
+@pytest.mark.parametrize("half", [1, 2, 3, 4, 7, 24])
+def test_row_widths_of_the_operator_kernels(gpu, n, half):
+    """One FP64 V-cycle on rows of 3 to 49 entries, tiles with a last partial warp or one row more
+    than a block. In the oracle's order (SELL throughout, one row at a time and the next row loaded
+    ahead) bit for bit; by default and with lane groups throughout (wide_row) the row sums differ
+    in order: a few hundred additions deep over all levels, each within EPS of its magnitude."""
+    cb = gpu
+    own, nei, up, lo, diag, src = _banded(n, half)
+    ds = cb.DeviceSolver(cb.build_csr_pattern(n, own, nei))
+    settings = cb.AmgSettings(strength_threshold=0.04, coarse_size=16)
+    a = _csr(n, own, nei, diag, up, lo)
+    h = O.Hierarchy(a, theta=0.04, coarse_size=16)
+    ds.setup_amg(diag, up, lo, settings)
+    r = np.random.default_rng(8).standard_normal(n)
+    zr = O.vcycle_apply(h.a, h.p, h.r, h.coarse_inverse, r, 2, 0.7)
+    x = np.zeros(n)
+    ds.set_ordered(True)
+    for pair in (0, 1):
+        ds.set_tuning(cb.Tuning(vcycle_pair=pair))
+        ds.solve(diag, up, lo, src, x, cb.Method.Cg, True, cb.SolveControl(1e300, 1))
+        assert np.array_equal(ds.apply_amg(r), zr)
+    ds.set_ordered(False)
+    for t in (cb.Tuning(), cb.Tuning(wide_row=2), cb.Tuning(wide_row=2, lanes_div=4)):
+        ds.set_tuning(t)
+        ds.solve(diag, up, lo, src, x, cb.Method.Cg, True, cb.SolveControl(1e300, 1))
+        z = ds.apply_amg(r)
+        assert np.linalg.norm(z - zr) <= 1e3 * EPS * np.linalg.norm(zr)
+    ds.close()
+
+
+@pytest.mark.parametrize("half", [2, 3, 4, 9])
+def test_norms_of_the_ldu_solve_by_row_width(gpu, half):
+    """Residual and reference norms summed on the SELL operator: rows of 5, 7, 9 and 19 entries. All
+    terms are positive, so the two orders of the sums differ by less than n EPS of the result."""
+    cb = gpu
+    n = 3001
+    own, nei, up, lo, diag, src = _banded(n, half)
+    ds = cb.DeviceSolver(cb.build_csr_pattern(n, own, nei))
+    x = np.random.default_rng(4).standard_normal(n)
+    want = O.normalised_residual(own, nei, diag, up, lo, src, x)
+    r = ds.solve_ldu(diag, up, lo, src, x, cb.LduSettings(tolerance=1e-12, rel_tolerance=1e-6),
+                     cb.AmgSettings(strength_threshold=0.04))
+    assert abs(r.initial_residual - want) <= n * EPS * want
+    ds.close()
+
+
+@pytest.mark.parametrize("tiles", [1, 31, 32, 33, 444, 1184, 0])
+def test_reductions_over_any_number_of_tiles(gpu, tiles):
+    """Level-0 sums over one tile, the 32 that one warp adds in order, whole waves, and more than one
+    group (0: 2050 tiles of 256 rows, the last of one row): CG and BiCGStab to 1e-10 and the
+    norms of solve_ldu. The sums differ in order only: iterations within 1 (2), residuals at the
+    target."""
+    cb = gpu
+    n = 2049 * 256 + 1
+    own, nei, up, lo, diag, src = _banded(n, 1)
+    diag = diag + 1.0
+    ds = cb.DeviceSolver(cb.build_csr_pattern(n, own, nei))
+    ds.set_tuning(cb.Tuning(target_tiles=tiles))
+    a = _csr(n, own, nei, diag, up, lo)
+    tol = 1e-10 * np.linalg.norm(src)
+    xo, so = O.krylov(a, src, method=0, abs_tol=tol, max_iterations=500)
+    x = np.zeros(n)
+    st = ds.solve(diag, up, lo, src, x, cb.Method.Cg, False, cb.SolveControl(tol, 500))
+    assert st.converged and abs(st.iterations - so["iterations"]) <= 1
+    assert np.linalg.norm(src - a.matvec(x)) <= 1.05 * tol
+    xb = np.zeros(n)
+    xo, so = O.krylov(a, src, method=1, abs_tol=tol, max_iterations=500)
+    st = ds.solve(diag, up, lo, src, xb, cb.Method.BiCgStab, False, cb.SolveControl(tol, 500))
+    assert st.converged and abs(st.iterations - so["iterations"]) <= 2
+    assert np.linalg.norm(src - a.matvec(xb)) <= 1.05 * tol
+    want = O.normalised_residual(own, nei, diag, up, lo, src, x)
+    r = ds.solve_ldu(diag, up, lo, src, x, cb.LduSettings(tolerance=1.0))
+    # x is nearly the solution: the residual itself carries the cancellation of b - A x
+    assert r.iterations == 0 and abs(r.initial_residual - want) <= 1e-4 * want
+    ds.close()
+
+
+@pytest.mark.parametrize("max_it", [1, 2, 3])
+def test_bicgstab_limit_and_half_step(gpu, max_it):
+    """The iteration limit is reported as the oracle reports it; a diagonal matrix is solved by the
+    first half step."""
+    cb = gpu
+    case = W.cavity(8)
+    up, lo, diag, src = _pressure(case)
+    a = _csr(case.n, case.owner, case.neighbour, diag, up, lo)
+    ds = cb.DeviceSolver(cb.build_csr_pattern(case.n, case.owner, case.neighbour))
+    tol = 1e-10 * np.linalg.norm(src)
+    xo, so = O.krylov(a, src, method=1, abs_tol=tol, max_iterations=max_it)
+    x = np.zeros(case.n)
+    st = ds.solve(diag, up, lo, src, x, cb.Method.BiCgStab, False, cb.SolveControl(tol, max_it))
+    assert not st.converged and st.iterations == so["iterations"] == max_it
+    # three iterations from the same start: sums of 512 terms in another order, not yet amplified
+    assert np.linalg.norm(x - xo) <= 1e-9 * np.linalg.norm(xo)
+    z = np.zeros_like(up)
+    d = 4.0 * np.ones(case.n)
+    xd = np.zeros(case.n)
+    st = ds.solve(d, z, z, src, xd, cb.Method.BiCgStab, False, cb.SolveControl(tol, max_it))
+    assert st.converged and st.iterations == 1
+    assert np.linalg.norm(src - d * xd) <= tol
+    ds.close()
+
+
+@pytest.mark.parametrize("tol", [1e-6, 1e-12, 1e-18])
+def test_mixed_precision_reports_the_checked_residual(gpu, tol):
+    """Mixed precision: a system at its target is checked in FP64 and goes on if the check fails.
+    `converged` and `true_residual` are those of the returned x, also where the target is out of
+    reach."""
+    cb = gpu
+    case = W.tet(8)
+    up, lo, diag, src = _pressure(case)
+    a = _csr(case.n, case.owner, case.neighbour, diag, up, lo)
+    ds = cb.DeviceSolver(cb.build_csr_pattern(case.n, case.owner, case.neighbour))
+    ds.set_precision(cb.Precision.MIXED)
+    ds.setup_amg(diag, up, lo, cb.AmgSettings(strength_threshold=0.04, coarse_size=50))
+    t = tol * np.linalg.norm(src)
+    x = np.zeros(case.n)
+    st = ds.solve(diag, up, lo, src, x, cb.Method.Cg, True, cb.SolveControl(t, 60))
+    got = np.linalg.norm(src - a.matvec(x))
+    mag = np.linalg.norm(np.abs(src) + _abs_matvec(a, x))
+    assert abs(got - st.true_residual) <= 64 * EPS * mag
+    assert st.iterations <= 60
+    if st.converged:
+        assert st.true_residual <= t
+    assert st.converged or tol < 1e-15
+    ds.close()
+
+
+def _abs_matvec(a, x):
+    return np.add.reduceat(np.abs(a.va) * np.abs(x)[a.ci], a.rp[:-1])
+
+
+@pytest.mark.parametrize("n", [4095, 4097, 9000])
+@pytest.mark.parametrize("half", [3, 4, 7, 8, 9, 10, 15, 16])
+def test_setup_at_the_row_lengths_of_its_kernels(gpu, n, half):
+    """Rows of 2 half + 1 entries: products of 7 to 33 contributions (8, 16 and 32 lanes, then
+    tables), sorts of up to 32 entries and more, aggregation of levels around 4096 rows and 20
+    strong entries a row. Every level equals the host build bit for bit."""
+    cb = gpu
+    own, nei, up, lo, diag, _ = _banded(n, half, seed=half)
+    a = _csr(n, own, nei, diag, up, lo)
+    view = cb.CsrView(a.n_rows, a.rp, a.ci, a.va)
+    for theta in (0.0, 0.02):
+        s = cb.AmgSettings(strength_threshold=theta)
+        d, h = cb.AmgHierarchy(view, s, device=True), cb.AmgHierarchy(view, s)
+        assert d.levels() == h.levels()
+        for l in range(h.levels()):
+            pairs = [(d.level_matrix(l), h.level_matrix(l))]
+            if l + 1 < h.levels():
+                assert np.array_equal(d.aggregates(l)[0], h.aggregates(l)[0])
+                pairs += [(d.level_prolongation(l), h.level_prolongation(l)),
+                          (d.level_restriction(l), h.level_restriction(l))]
+            for g, w in pairs:
+                assert np.array_equal(g.row_ptr, w.row_ptr) and np.array_equal(g.col, w.col)
+                assert np.array_equal(g.val, w.val)
+        assert np.array_equal(d.coarse_inverse(), h.coarse_inverse())
+
+
+@pytest.mark.parametrize("n,nc", [(6, 2), (96, 32), (1248, 416), (1251, 417), (1500, 500)])
+def test_dense_coarse_solve_by_size(gpu, n, nc):
+    """Two levels: the dense inverse's rows up to 13 x 32 entries are loaded ahead, the rest behind
+    them. Bit for bit in the oracle's order, else sums of nc terms in another order."""
+    cb = gpu
+    own, nei, up, lo, diag, src = _banded(n, 1)
+    a = _csr(n, own, nei, diag, up, lo)
+    h = O.Hierarchy(a, theta=0.04, max_levels=2, coarse_size=3)
+    assert h.levels == 2 and h.a[1].n_rows == nc
+    ds = cb.DeviceSolver(cb.build_csr_pattern(n, own, nei))
+    ds.setup_amg(diag, up, lo, cb.AmgSettings(strength_threshold=0.04, max_levels=2, coarse_size=3))
+    r = np.random.default_rng(8).standard_normal(n)
+    zr = O.vcycle_apply(h.a, h.p, h.r, h.coarse_inverse, r, 2, 0.7)
+    for ordered in (True, False):
+        ds.set_ordered(ordered)
+        x = np.zeros(n)
+        ds.solve(diag, up, lo, src, x, cb.Method.Cg, True, cb.SolveControl(1e300, 1))
+        z = ds.apply_amg(r)
+        assert np.linalg.norm(z - zr) <= (0.0 if ordered else nc * EPS * np.linalg.norm(zr))
+    ds.close()
