@@ -339,6 +339,19 @@ int csr_lanes(double rows, double avg, int lanes_div, bool fp64) {
     return lanes;
 }
 
+// Level-0 Krylov tiles for a target of `target` CTAs: whole waves of the CTAs that the SpMV kernels
+// keep resident, so that no wave is left nearly empty, and as few waves as tiles of at most 4096
+// rows allow (a thread streams its rows; each tile ends in a ticket). Solves on 1184 tiles (2.7
+// waves of 7-entry rows, or one and a few CTAs) against this rule: graded 885K cells FP64 5.22
+// against 4.95 ms, 176K cells mixed 1.29 against 1.19, scalar step (BiCGStab, 512K cells) 1.15
+// against 0.98, 304K tets mixed 1.81 against 1.73. 5.1M tets (8690 rows a tile in one wave): 11.63
+// ms in one wave, 11.35 in two, 11.53 in three.
+int krylov_tiles(int rows, int visit, int target) {
+    const int wave = 148 * krylov_ctas(visit);
+    if (target <= wave) return target;
+    return wave * std::min(target / wave, ceil_div(rows, 4096 * wave));
+}
+
 int grid_of(long long n) { return static_cast<int>(std::max<long long>(1, (n + 255) / 256)); }
 
 } // namespace
@@ -478,13 +491,17 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
     off0_.resize(n_sys_);
     for (int s = 0; s < n_sys_; ++s) off0_[s] = off[0][s];
     cudaStream_t st = stream_;
-    // Krylov tiles of level 0 (the reductions): kSellRows rows, or a fixed tile count when
-    // target_tiles > 0; coarser levels use their operators' own tiles
+    // Krylov tiles of level 0 (the reductions): kSellRows rows, or a tile count when target_tiles > 0;
+    // coarser levels use their operators' own tiles
     std::vector<int> sys_tile0(n_sys_ + 1, 0);
+    double nnz0 = 0.0;
+    for (const SystemSpec& sp : systems) nnz0 += sp.rp[sp.n];
     for (int l = 0; l < 1; ++l) {
         DevLevel& d = lv_[l];
+        const int rows0 = std::max(d.n_rows, 1);
+        const int visit0 = krylov_visit_of(nnz0 / rows0, tuning_.krylov_pair != 0);
         const int base = tuning_.target_tiles > 0
-                             ? std::max(kSellRows, round_up(ceil_div(std::max(d.n_rows, 1), tuning_.target_tiles), kSellRows))
+                             ? std::max(kSellRows, round_up(ceil_div(rows0, krylov_tiles(rows0, visit0, tuning_.target_tiles)), kSellRows))
                              : kSellRows;
         std::vector<int> trow, tsys;
         int nc_tiles = -1;

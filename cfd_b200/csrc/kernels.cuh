@@ -631,6 +631,16 @@ __host__ __device__ inline int krylov_visit_of(double width, bool ahead) {
     return ahead ? kVisitStream7 : kVisitSell7;
 }
 
+// CTAs per SM of the level-0 Krylov kernels.
+inline int krylov_ctas(int visit) {
+    switch (visit) {
+    case kVisitStream5: return kMinBlocks<double, kVisitStream5, false>;
+    case kVisitStream7: return kMinBlocks<double, kVisitStream7, false>;
+    case kVisitSell5: return kMinBlocks<double, kVisitSell5, false>;
+    default: return kMinBlocks<double, kVisitSell7, false>;
+    }
+}
+
 // Tile bookkeeping shared by all tiled kernels.
 struct TileCtx {
     int tile, s, r0, r1;
