@@ -531,7 +531,13 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
         // 512 rows: residual 52.6 / 50.3 us, prolongation 40.6 / 37.5 us; on 885K rows no gain
         const int rows_all = lv_[static_cast<size_t>(row_level)].n_rows;
         const int factor = rows_all > 8 * 148 * 8 * kSellRows ? 2 : 1;
-        const int rpt = fmt == kFmtSell ? factor * std::max(kSellRows, tuning_.sell_rows / kSellRows * kSellRows) : kBlock / fmt;
+        // FP64 rows of more than 5 entries: CTAs of half the threads, since the register limit leaves four
+        // to six CTAs of 256 on an SM and a CTA frees its place only with its longest row. FP64 solves
+        // by 256 / 128 (64) threads: graded 1.7M cells 12.37 / 12.04 ms, 885K 4.93 / 4.90 (5.01), 343K
+        // 2.19 / 2.12, cavity 32K 0.625 / 0.619 (0.635); 5-entry rows no gain, FP32 1 % slower.
+        m.threads = kBlock;
+        if (fmt == kFmtSell && tuning_.vcycle_pair == 0 && !need32_ && row_width(m) > 5.25) m.threads = kBlock / 2;
+        const int rpt = fmt == kFmtSell ? factor * std::max(1, tuning_.sell_rows / kSellRows) * m.threads : kBlock / fmt;
         std::vector<int> trow, tsys;
         int n_nc = -1, end = 0;
         for (int k = 0; k < n_sys_; ++k) {
@@ -1347,10 +1353,11 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
     struct Launch {
         Tiles first;
         int second; // grid
+        int threads; // of a CTA
         int visit;  // row-visiting strategy of the operator's kernels
     };
     auto TL = [&](int, const DevSell64_32& m, bool nc) -> Launch {
-        return {m.tiles, nc ? m.n_tiles_nc : m.n_tiles, vcycle_visit(m)};
+        return {m.tiles, nc ? m.n_tiles_nc : m.n_tiles, m.threads, vcycle_visit(m)};
     };
     std::vector<T*> cur(L, nullptr);
     // levels lt and below run in the persistent tail kernel when its phases are prepared
@@ -1375,8 +1382,8 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
             T* c = start;
             for (int k = 1; k < sweeps_; ++k) {
                 T* o = c == x ? y : x;
-                if (l == 0) with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
-                else with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
+                if (l == 0) with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, ta.threads, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
+                else with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, ta.threads, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
                 mark("smooth", l, spmv_b(d.a, n, n) + sv * n + sb * n);
                 c = o;
             }
@@ -1384,30 +1391,30 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
         } else {
             const auto ta = TL(l, d.a, true);
             if (l == 0) {
-                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_first<T, double, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), r_, start, fuse); });
+                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_first<T, double, decltype(V)::value>, ta.second, ta.threads, 0, s, A(l), ta.first, stv, WD(l), r_, start, fuse); });
             } else {
-                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_first<T, T, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), Bv(l), start, fuse); });
+                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_first<T, T, decltype(V)::value>, ta.second, ta.threads, 0, s, A(l), ta.first, stv, WD(l), Bv(l), start, fuse); });
             }
             mark("smooth_first", l, fuse ? spmv_b(d.a, n, n) - sv * n + sv * n + sb * n : 2.0 * sv * n + sb * n);
             T* c = start;
             for (int k = fuse ? 2 : 1; k < sweeps_; ++k) {
                 T* o = c == x ? y : x;
-                if (l == 0) with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
-                else with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
+                if (l == 0) with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, ta.threads, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
+                else with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, ta.threads, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
                 mark("smooth", l, spmv_b(d.a, n, n) + sv * n + sb * n);
                 c = o;
             }
             cur[l] = c;
         }
         const auto tr = TL(l, d.a, true);
-        if (l == 0) with_visit(tr.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_residual<T, double, decltype(V)::value>, tr.second, kBlock, 0, s, A(l), tr.first, stv, r_, cur[l], Tv(l)); });
-        else with_visit(tr.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_residual<T, T, decltype(V)::value>, tr.second, kBlock, 0, s, A(l), tr.first, stv, Bv(l), cur[l], Tv(l)); });
+        if (l == 0) with_visit(tr.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_residual<T, double, decltype(V)::value>, tr.second, tr.threads, 0, s, A(l), tr.first, stv, r_, cur[l], Tv(l)); });
+        else with_visit(tr.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_residual<T, T, decltype(V)::value>, tr.second, tr.threads, 0, s, A(l), tr.first, stv, Bv(l), cur[l], Tv(l)); });
         mark("residual", l, spmv_b(d.a, n, n) + sb * n);
         const DevLevel& nx = lv_[l + 1];
         const auto tq = TL(l + 1, d.r, false);
         const bool next_x1 = x1_by_restrict && l + 2 < L && nx.n_rows_nc > 0;
         with_visit(tq.visit, [&](auto V) {
-            launch_k(tuning_.pdl != 0, k_vc_spmv<T, decltype(V)::value>, tq.second, kBlock, 0, s, 
+            launch_k(tuning_.pdl != 0, k_vc_spmv<T, decltype(V)::value>, tq.second, tq.threads, 0, s, 
                 R(l), tq.first, stv, Tv(l), Bv(l + 1), next_x1 ? WD(l + 1) : nullptr,
                 next_x1 ? start_buffer<T>(l + 1) : nullptr, next_x1 ? nx.n_rows_nc : 0);
         });
@@ -1440,7 +1447,7 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
         T* c = cur[l];
         const auto tp = TL(l, d.p, true);
         with_visit(tp.visit, [&](auto V) {
-            launch_k(tuning_.pdl != 0, k_vc_prolong<T, decltype(V)::value>, tp.second, kBlock, 0, s, P(l), tp.first, stv, X(l + 1), c);
+            launch_k(tuning_.pdl != 0, k_vc_prolong<T, decltype(V)::value>, tp.second, tp.threads, 0, s, P(l), tp.first, stv, X(l + 1), c);
         });
         const auto ta = TL(l, d.a, true);
         mark("prolong", l, spmv_b(d.p, n, lv_[l + 1].n_rows) + sv * n);
@@ -1454,10 +1461,10 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
                 });
                 mark("smooth_dot", l, spmv_b(d.a, n, n) + sv * n + sb * n + (flexible ? 8.0 * n : 0.0));
             } else if (l == 0) {
-                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
+                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, ta.second, ta.threads, 0, s, A(l), ta.first, stv, WD(l), r_, c, o); });
                 mark("smooth", l, spmv_b(d.a, n, n) + sv * n + sb * n);
             } else {
-                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, kBlock, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
+                with_visit(ta.visit, [&](auto V) { launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, ta.second, ta.threads, 0, s, A(l), ta.first, stv, WD(l), Bv(l), c, o); });
                 mark("smooth", l, spmv_b(d.a, n, n) + sv * n + sb * n);
             }
             c = o;
@@ -1886,12 +1893,12 @@ double Engine::time_sweep(int level, int reps, double* bytes) {
         }
         with_visit(visit, [&](auto V) {
             if (level == 0) {
-                launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, grid, kBlock, 0, stream_, op, tiles, nullptr, wd, r_, x, y);
+                launch_k(tuning_.pdl != 0, k_vc_jacobi<T, double, decltype(V)::value>, grid, m.threads, 0, stream_, op, tiles, nullptr, wd, r_, x, y);
             } else {
                 const T* bv;
                 if constexpr (sizeof(T) == 8) bv = d.b64;
                 else bv = d.b32;
-                launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, grid, kBlock, 0, stream_, op, tiles, nullptr, wd, bv, x, y);
+                launch_k(tuning_.pdl != 0, k_vc_jacobi<T, T, decltype(V)::value>, grid, m.threads, 0, stream_, op, tiles, nullptr, wd, bv, x, y);
             }
         });
     };

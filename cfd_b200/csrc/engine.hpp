@@ -193,9 +193,10 @@ private:
         long long slots = 0;  // stored entries (SELL: with padding)
         long long nnz = 0;    // algorithmic nonzeros
         int max8_slots = 0;   // SELL: most slots of any 8 consecutive slices (a staged chunk)
-        // launch tiles of the operator's own row space, 256 threads each: sell_rows rows (SELL) or
+        // launch tiles of the operator's own row space: sell_rows / 256 rows a thread (SELL) or
         // 256 / G rows (CSR)
         Tiles tiles{};
+        int threads = kBlock; // of a CTA
         int n_tiles = 0;
         int n_tiles_nc = 0;   // tiles of systems that continue to a coarser level
     };
@@ -231,7 +232,7 @@ private:
         const bool fp64 = m.s64.val != nullptr;
         const int fmt = fp64 ? m.s64.fmt : m.s32.fmt;
         if (fmt == kFmtSell && tuning_.vcycle_pair) return krylov_visit_of(row_width(m), true);
-        return visit_of(fmt, row_width(m), m.n_tiles, fp64 && !need32_);
+        return visit_of(fmt, row_width(m), static_cast<int>(static_cast<long long>(m.n_tiles) * m.threads / kBlock), fp64 && !need32_);
     }
     // stored entries per row of a SELL operator
     static double row_width(const DevSell64_32& m) {

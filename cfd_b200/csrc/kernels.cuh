@@ -567,7 +567,7 @@ template <int V, class T> struct Visit {
             for (int pos = r0 + static_cast<int>(threadIdx.x); pos < r1;) {
                 const auto e = pre(r.row);
                 f(r.row, sell_sum<kAhead, B>(m, r, v, c, xa), e);
-                pos += kBlock;
+                pos += static_cast<int>(blockDim.x);
                 if (pos < r1) {
                     r = sell_row_at(m, pos);
                     sell_load<B>(m, r.k, r.e, r.base, v, c);

@@ -160,8 +160,8 @@ typedef struct cfdb_hierarchy cfdb_hierarchy;
 int cfdb_amg_setup(const cfdb_csr* a, const cfdb_amg_settings* settings,
                    cfdb_hierarchy** out);
 /* The same hierarchy built on the device (sparse products, strength graph, transfers and
- * Galerkin operators in CUDA kernels; the sequential aggregation on the host), bit-identical
- * to cfdb_amg_setup. */
+ * Galerkin operators in CUDA kernels; the aggregation too, except on small or dense levels and
+ * where many rows are left for its third pass), bit-identical to cfdb_amg_setup. */
 int cfdb_amg_setup_device(const cfdb_csr* a, const cfdb_amg_settings* settings,
                           cfdb_hierarchy** out);
 int cfdb_hierarchy_destroy(cfdb_hierarchy* h);
@@ -379,7 +379,7 @@ int cfdb_system_apply_amg(cfdb_system* sys, const double* r, double* z);
  * (slower on wide coarse levels). Default off: wide coarse rows use warp-per-row sums. */
 int cfdb_system_set_ordered(cfdb_system* sys, int ordered);
 
-/* Per-kernel device time of the initial preconditioning plus one iteration (events around
+/* Per-kernel device time of the initial residual plus one iteration (events around
  * every kernel, averaged over reps after one warm-up), with each kernel's algorithmic bytes. */
 typedef struct {
     char name[32];
@@ -430,8 +430,9 @@ typedef struct {
     int lanes_div;    /* lanes per CSR row ~ 4 x average row length / lanes_div (4..256, within about a
                          wave of threads per operator), default 16 */
     int fuse_first;   /* first two smoothing sweeps in one kernel, default 0 */
-    int sell_rows;    /* rows per CTA of SELL operators (one row per thread per pass): a multiple
-                         of 256, default 256 */
+    int sell_rows;    /* rows per CTA of 256 threads of SELL operators (one row per thread per pass;
+                         smaller CTAs and larger operators in proportion): a multiple of 256,
+                         default 256 */
     int krylov_pair;  /* level-0 Krylov SpMV kernels load a thread's next row while they sum the current
                          one (1, default), or take one row at a time (0) */
     int tail_rows;    /* coarse levels of at most this many rows, with all coarser ones, run as one
