@@ -5,7 +5,7 @@
 // r0.r, the pp / ph / v / s / sh / t updates, omega = (t.s) / (t.t) or 0, the early exit on
 // |s| and the exits on rho == 0, omega == 0 and r0.v == 0; iterations capped at the maximum).
 // Every update rounds each product and sum separately in the reference's operand order. Dot
-// products are the two-level tile reductions of the CG kernels (reproducible; they differ from
+// products are the tile reductions of the CG kernels (reproducible; they differ from
 // the reference's sequential sums only in summation order).
 //
 // The scalars live on the device (BcgState): each dot product is part of the kernel that makes
@@ -311,7 +311,7 @@ SolveResult Engine::solve_bicgstab(const SolveRequest& rq, bool want_true) {
         SysState cg;
         int words[2];
     };
-    Upload* h = static_cast<Upload*>(h_state_.get(sizeof(Upload)));
+    Upload* h = static_cast<Upload*>(host_state(sizeof(Upload)));
     h->s = BcgState{};
     h->s.tol = rq.tol;
     h->s.max_it = rq.max_it;

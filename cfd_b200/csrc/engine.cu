@@ -359,8 +359,16 @@ int grid_of(long long n) { return static_cast<int>(std::max<long long>(1, (n + 2
 Engine::Engine(int device) : device_(device) {
     CFDB_CUDA(cudaSetDevice(device));
     CFDB_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-    CFDB_CUDA(cudaHostAlloc(&progress_, sizeof(Progress), cudaHostAllocMapped | cudaHostAllocPortable));
+    void* block = nullptr;
+    CFDB_CUDA(cudaHostAlloc(&block, kHostBlock, cudaHostAllocMapped | cudaHostAllocPortable));
+    progress_ = static_cast<Progress*>(block);
     *progress_ = Progress{};
+}
+
+void* Engine::host_state(size_t bytes) {
+    constexpr size_t kOff = 256; // behind the progress record
+    static_assert(sizeof(Progress) <= kOff);
+    return bytes <= kHostBlock - kOff ? reinterpret_cast<char*>(progress_) + kOff : static_cast<char*>(h_state_.get(bytes));
 }
 
 Engine::~Engine() {
@@ -1777,7 +1785,7 @@ std::vector<SolveResult> Engine::solve(Mode mode, const std::vector<SolveRequest
     if (mode == Mode::AmgMixed && !need32_) fail(5, "solve: mixed precision needs the FP32 hierarchy");
     if (mode == Mode::AmgFp64 && !need64_) fail(5, "solve: FP64 AMG needs the FP64 hierarchy");
     const size_t st_bytes = sizeof(SysState) * static_cast<size_t>(n_sys_) + 2 * sizeof(int);
-    SysState* hs = static_cast<SysState*>(h_state_.get(st_bytes));
+    SysState* hs = static_cast<SysState*>(host_state(st_bytes));
     int max_it = 0;
     for (int s = 0; s < n_sys_; ++s) {
         SysState& t = hs[rank_[s]];

@@ -305,9 +305,15 @@ private:
     int* n_active_ = nullptr; // behind the systems' states: one upload starts a solve
     int* error_ = nullptr;
     int* seq_ = nullptr;           // device count of published records
-    Progress* progress_ = nullptr; // page-locked, mapped: the last record
+    // Page-locked, mapped: the last record, and behind it the image of the states and the two words
+    // behind them (host_state; h_state_ where many systems need more). One small block made with the
+    // engine: page-locking a megabyte costs milliseconds, which a first solve should not pay (a new
+    // system's first solve of the box of 16^3 cells: 2.4 to 5.3 ms with it, 0.9 without).
+    static constexpr size_t kHostBlock = 16 << 10;
+    Progress* progress_ = nullptr;
+    void* host_state(size_t bytes);
     int published_ = 0;            // records published by the work launched so far
-    PinnedBuffer h_state_;         // page-locked image of the states and the two words behind them
+    PinnedBuffer h_state_;
     // coarse blocks
     int n_blocks_ = 0;
     int n_single_ = 0;        // systems whose hierarchy has one level (Jacobi-preconditioned CG)

@@ -107,7 +107,7 @@ LduNorms Engine::residual_norms() {
     else
         launch_k(pdl, k_ldu_norms<7>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, n, b_, x_, red_, red2_, norms_);
     launches_ += 2;
-    NormState* h = static_cast<NormState*>(h_state_.get(sizeof(NormState)));
+    NormState* h = static_cast<NormState*>(host_state(sizeof(NormState)));
     CFDB_CUDA(cudaMemcpyAsync(h, norms_, sizeof(NormState), cudaMemcpyDeviceToHost, stream_));
     CFDB_CUDA(cudaStreamSynchronize(stream_));
     return LduNorms{h->res, h->norm, h->r2};
