@@ -3,8 +3,8 @@
 // Per level (amg.cpp:122-190, in the host build's rounding order):
 //   d      last diagonal entry of each row (amg.cpp:82-92)
 //   S      strength graph: i != j and |a_ij| > theta sqrt|d_i d_j| (amg.cpp:22-27)
-//   agg    aggregation passes 1-2 on the device (k_seed_sweep, k_pass2); a level with rows left
-//          for pass 3 is read back and aggregated on the host (amg.cpp:12-78)
+//   agg    aggregation passes 1-3 on the device (k_seed_sweep, k_pass2, k_pass3); small or dense levels and
+//          those with many rows left for pass 3 are aggregated on the host (amg.cpp:12-78)
 //   inv    1/d or 0; rho = max_i |inv_i| sum_j |a_ij|; omega = 4 / (3 rho) (amg.cpp:150-166)
 //   C      (D^-1 A) P_tent: row i accumulates inv_i a_ik into column agg(k), k ascending
 //   P      P_tent - omega C over the union pattern, exact zeros dropped (amg.cpp:168-172)
@@ -1431,8 +1431,12 @@ bool device_aggregation(int n, long long ns) { return n >= 4096 && ns <= 20LL * 
 // conflict lists pass 2^31 entries: the caller then aggregates on the host.
 int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, int* agg) {
     cudaStream_t st = cx.st;
+    // scratch of its own (the transpose, conflict lists), given back before the products need theirs;
+    // every path out of here has synchronised st
+    Scratch own;
     Ctx tx = cx;
-    tx.keep = nullptr; // the transpose is scratch
+    tx.mem = &own;
+    tx.keep = nullptr;
     DevCsr g;
     g.n_rows = g.n_cols = n;
     g.nnz = ns;
@@ -1440,20 +1444,20 @@ int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, in
     g.ci = sci;
     g.va = sav;
     const DevCsr t = transpose(tx, g);
-    int* state = cx.mem->alloc<int>(n);
+    int* state = tx.mem->alloc<int>(n);
     int* counter = cx.d_counts + kClasses + kTinyClasses; // the spare counter
     k_seed_init<<<grid_for(n), kThreads, 0, st>>>(n, srp, state);
-    int* ccnt = cx.mem->alloc<int>(static_cast<size_t>(n) + 1);
-    int* crp = cx.mem->alloc<int>(static_cast<size_t>(n) + 1);
+    int* ccnt = tx.mem->alloc<int>(static_cast<size_t>(n) + 1);
+    int* crp = tx.mem->alloc<int>(static_cast<size_t>(n) + 1);
     k_conflicts<false><<<grid_for(n), kThreads, 0, st>>>(n, srp, sci, t.rp, t.ci, ccnt, nullptr, nullptr);
-    const long long n_conf = scan(cx, ccnt, n, crp);
+    const long long n_conf = scan(tx, ccnt, n, crp);
     if (n_conf > INT_MAX) return -1;
-    int* cci = cx.mem->alloc<int>(static_cast<size_t>(n_conf));
+    int* cci = tx.mem->alloc<int>(static_cast<size_t>(n_conf));
     k_conflicts<true><<<grid_for(n), kThreads, 0, st>>>(n, srp, sci, t.rp, t.ci, nullptr, crp, cci);
     int* at = ccnt; // conflicts passed so far
     CFDB_CUDA(cudaMemsetAsync(at, 0, sizeof(int) * static_cast<size_t>(n), st));
     // lo of each sweep of a batch; lo[0] = 0, then the last lo of the previous batch
-    int* lo = cx.mem->alloc<int>(kSeedBatch + 1);
+    int* lo = tx.mem->alloc<int>(kSeedBatch + 1);
     CFDB_CUDA(cudaMemsetAsync(lo, 0, sizeof(int), st));
     const int grid = grid_for(std::min(n, kSeedWindow));
     for (long long sweeps = 0;;) {
@@ -1470,11 +1474,11 @@ int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, in
         if (last >= n) break;
         CFDB_CUDA(cudaMemcpyAsync(lo, lo + kSeedBatch, sizeof(int), cudaMemcpyDeviceToDevice, st));
     }
-    int* flag = cx.mem->alloc<int>(static_cast<size_t>(n) + 1);
-    int* id = cx.mem->alloc<int>(static_cast<size_t>(n) + 1);
+    int* flag = tx.mem->alloc<int>(static_cast<size_t>(n) + 1);
+    int* id = tx.mem->alloc<int>(static_cast<size_t>(n) + 1);
     k_seed_flags<<<grid_for(n), kThreads, 0, st>>>(n, state, flag);
-    const long long n_seeds = scan(cx, flag, n, id);
-    int* agg1 = cx.mem->alloc<int>(n);
+    const long long n_seeds = scan(tx, flag, n, id);
+    int* agg1 = tx.mem->alloc<int>(n);
     k_pass1_cover<<<grid_for(n), kThreads, 0, st>>>(n, t.rp, t.ci, state, id, agg1);
     CFDB_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), st));
     k_pass2<<<grid_for(n), kThreads, 0, st>>>(n, srp, sci, sav, agg1, agg, counter);
@@ -1483,10 +1487,10 @@ int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, in
     CFDB_CUDA(cudaMemcpyAsync(&left, counter, sizeof(int), cudaMemcpyDeviceToHost, st));
     sync(st);
     if (left > 0 && left <= kPass3Device) {
-        int* pos = cx.mem->alloc<int>(static_cast<size_t>(n) + 1);
-        int* list = cx.mem->alloc<int>(left);
+        int* pos = tx.mem->alloc<int>(static_cast<size_t>(n) + 1);
+        int* list = tx.mem->alloc<int>(left);
         k_left_flags<<<grid_for(n), kThreads, 0, st>>>(n, agg, flag);
-        scan(cx, flag, n, pos);
+        scan(tx, flag, n, pos);
         k_left_list<<<grid_for(n), kThreads, 0, st>>>(n, agg, pos, list);
         int n_agg = static_cast<int>(n_seeds);
         CFDB_CUDA(cudaMemcpyAsync(counter, &n_agg, sizeof(int), cudaMemcpyHostToDevice, st));

@@ -4,8 +4,8 @@
 // restriction, Galerkin products, zero pruning) runs in device kernels. The aggregation
 // (amg.cpp:12-78) is a sequence of greedy passes whose result depends on the visiting order:
 // passes 1 and 2 run on the device with the sequential result (pass 1 as the lexicographically
-// first independent set it is, resolved by sweeps); a level that leaves rows for pass 3 is
-// aggregated on the host from its strength graph. Every product and
+// first independent set it is, resolved by sweeps over conflict lists; pass 3 by one thread where few
+// rows are left for it); other levels are aggregated on the host from their strength graph. Every product and
 // sum is rounded in the order the host build (amg_setup, host_algos.cpp) uses, so the device
 // hierarchy is bit-identical to it: aggregates, P, R, coarse operators and coarse inverse.
 #pragma once
