@@ -852,7 +852,7 @@ class DeviceSolver:
         _check(_lib.cfdb_system_set_ordered(self._h, 1 if ordered else 0))
 
     def profile(self, use_amg: bool = True, reps: int = 5) -> list:
-        """Per-kernel device time (ms) and algorithmic bytes of the initial preconditioning and
+        """Per-kernel device time (ms) and algorithmic bytes of the initial residual and
         one iteration, in launch order: [(name, level, ms, bytes), ...]."""
         recs = (KernelRecordStruct * 512)()
         n = C.c_int()
