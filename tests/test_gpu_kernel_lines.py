@@ -214,3 +214,29 @@ def test_dense_coarse_solve_by_size(gpu, n, nc):
         z = ds.apply_amg(r)
         assert np.linalg.norm(z - zr) <= (0.0 if ordered else nc * EPS * np.linalg.norm(zr))
     ds.close()
+
+
+@pytest.mark.parametrize("n_sys", [1, 167, 168, 300])
+def test_batches_around_the_state_block(gpu, n_sys):
+    """The states of up to 167 systems (96 bytes each) travel in the engine's page-locked block, more
+    in a buffer of their own: every system of a batch reaches its own target."""
+    import torch
+    cb = gpu
+    n = 24
+    own, nei, up, lo, diag, _ = _banded(n, 2)
+    a = _csr(n, own, nei, diag, up, lo)
+    rng = np.random.default_rng(n_sys)
+    b = cb.Batch([n] * n_sys, [len(own)] * n_sys, np.tile(own, n_sys), np.tile(nei, n_sys))
+    rep = lambda v: np.tile(v, n_sys)  # noqa: E731
+    src = rng.standard_normal(n * n_sys)
+    b.setup_amg(rep(diag), rep(up), rep(lo))
+    T = lambda v: torch.as_tensor(v, dtype=torch.float64, device="cuda")  # noqa: E731
+    x = torch.zeros(n * n_sys, dtype=torch.float64, device="cuda")
+    tol = [10.0 ** -(4 + k % 7) * np.linalg.norm(src[k * n:(k + 1) * n]) for k in range(n_sys)]
+    for _ in range(2):
+        x.zero_()
+        stats = b.solve_device(T(rep(diag)), T(rep(up)), T(rep(lo)), T(src), x, [cb.SolveControl(t, 100) for t in tol])
+        got = x.cpu().numpy()
+        for k in range(n_sys):
+            r = np.linalg.norm(src[k * n:(k + 1) * n] - a.matvec(got[k * n:(k + 1) * n]))
+            assert stats[k].converged and r <= 1.05 * tol[k]
