@@ -982,7 +982,7 @@ __global__ void k_row_len(int n, const int* __restrict__ rp, int* len) {
     if (i < n) len[i] = rp[i + 1] - rp[i];
 }
 
-// sorts rows of (ci, va) by ci; CAP > 0: in shared memory, else in device tables (gkeys/gvals)
+// sorts rows of (ci, va) by ci (entries of equal ci stay, in any order); CAP > 0: in shared memory, else in device tables (gkeys/gvals)
 template <int G, int CAP, int PER>
 __global__ void __launch_bounds__(G* PER) k_seg_sort(const int* __restrict__ rows, int n_list, const int* __restrict__ rp,
                                                       int* ci, double* va, const long long* goff, const int* gcap,
@@ -1006,13 +1006,17 @@ __global__ void __launch_bounds__(G* PER) k_seg_sort(const int* __restrict__ row
     const int r0 = rp[i], len = rp[i + 1] - r0;
     if (len > cap) return; // classified by length: cannot happen
     if constexpr (G == 32) {
-        // up to 32 entries: every lane counts the keys below its own and stores its entry there
+        // up to 32 entries: every lane counts the keys below its own, and those equal to it in front of it
+        // (a strength graph holds a column twice where its matrix does), and stores its entry there
         // (bitonic passes through shared memory took 226 us for 750K rows of 4 entries)
         if (len <= 32) {
             const int key = t < len ? ci[r0 + t] : kEmpty;
             const double v = t < len ? va[r0 + t] : 0.0;
             int at = 0;
-            for (int q = 0; q < len; ++q) at += __shfl_sync(0xffffffffu, key, q) < key ? 1 : 0;
+            for (int q = 0; q < len; ++q) {
+                const int other = __shfl_sync(0xffffffffu, key, q);
+                at += other < key || (other == key && q < t) ? 1 : 0;
+            }
             if (t < len) {
                 ci[r0 + at] = key;
                 va[r0 + at] = v;

@@ -240,3 +240,57 @@ def test_batches_around_the_state_block(gpu, n_sys):
         for k in range(n_sys):
             r = np.linalg.norm(src[k * n:(k + 1) * n] - a.matvec(got[k * n:(k + 1) * n]))
             assert stats[k].converged and r <= 1.05 * tol[k]
+
+
+def _scattered(n, per_row, seed):
+    """Symmetric, diagonally dominant CSR matrix of a sparse graph (two rows seldom share more than one
+    column) whose off-diagonal entries are each held twice with probability 1/2, the second copies at
+    the row's end."""
+    rng = np.random.default_rng(seed)
+    i = np.repeat(np.arange(n), per_row)
+    j = i + rng.integers(1, 400, len(i))
+    i, j = i[j < n], j[j < n]
+    pairs = np.unique(np.stack([i, j], 1), axis=0)
+    w = rng.uniform(0.5, 1.5, len(pairs))
+    rows = np.concatenate([pairs[:, 0], pairs[:, 1]])
+    cols = np.concatenate([pairs[:, 1], pairs[:, 0]])
+    vals = -np.concatenate([w, w])
+    diag = np.bincount(rows, -vals, n) + 0.05
+    rows, cols, vals = (np.concatenate([v, d]) for v, d in
+                        ((rows, np.arange(n)), (cols, np.arange(n)), (vals, diag)))
+    o = np.lexsort((cols, rows))
+    rows, cols, vals = rows[o], cols[o], vals[o]
+    twice = (rows != cols) & (rng.random(len(rows)) < 0.5)
+    r2 = np.concatenate([rows, rows[twice]])
+    c2 = np.concatenate([cols, cols[twice]])
+    v2 = np.concatenate([vals * np.where(twice, 0.625, 1.0), vals[twice] * 0.375])
+    o = np.argsort(r2, kind="stable")
+    rp = np.concatenate([[0], np.cumsum(np.bincount(r2, minlength=n))])
+    return rp.astype(np.int32), c2[o].astype(np.int32), v2[o]
+
+
+def _same_hierarchies(d, h):
+    assert d.levels() == h.levels()
+    for l in range(h.levels()):
+        pairs = [(d.level_matrix(l), h.level_matrix(l))]
+        if l + 1 < h.levels():
+            assert np.array_equal(d.aggregates(l)[0], h.aggregates(l)[0])
+            pairs += [(d.level_prolongation(l), h.level_prolongation(l)),
+                      (d.level_restriction(l), h.level_restriction(l))]
+        for g, w in pairs:
+            assert np.array_equal(g.row_ptr, w.row_ptr) and np.array_equal(g.col, w.col)
+            assert np.array_equal(g.val, w.val)
+    assert np.array_equal(d.coarse_inverse(), h.coarse_inverse())
+
+
+@pytest.mark.parametrize("n", [4095, 4096, 9000])
+@pytest.mark.parametrize("per_row", [1, 2, 4, 6, 12])
+def test_setup_with_repeated_columns(gpu, n, per_row):
+    """A CSR matrix whose rows (of about 4 to 40 entries) hold some columns twice: the device setup
+    treats them as separate entries, as the host build does, and equals it bit for bit, every time."""
+    cb = gpu
+    view = cb.CsrView(n, *_scattered(n, per_row, seed=per_row))
+    s = cb.AmgSettings(strength_threshold=0.0, max_levels=3)
+    h = cb.AmgHierarchy(view, s)
+    for _ in range(2):
+        _same_hierarchies(cb.AmgHierarchy(view, s, device=True), h)
