@@ -232,11 +232,14 @@ __device__ __forceinline__ void reduce_begin(int tile, int s, const Reduce& r) {
 }
 
 // Writes this tile's partials (reduce_begin has run); returns true in every thread of the system's
-// last CTA, whose thread 0 then holds the system totals in (a, b). ahead() runs in the last CTA's
+// last CTA, whose thread 0 then holds the system totals in (a, b). Every thread of a block of kBlock
+// calls it. The two flags are separate: no barrier lies between the block's reads of the first and
+// thread 0's write of the second (sum_pairs of up to 32 pairs has none), and a block may call this
+// twice, where the barriers of the next call's block_sum2 do lie between. ahead() runs in the last CTA's
 // thread 0 before the partials are summed: the loads of the scalar step that follows go there.
 template <class Ahead>
 __device__ __forceinline__ bool reduce_system(double& a, double& b, int tile, const Reduce& r, Ahead ahead) {
-    __shared__ int last;
+    __shared__ int last, last_group;
     block_sum2(a, b);
     const ReducePos p = reduce_pos();
     if (threadIdx.x == 0) {
@@ -255,11 +258,11 @@ __device__ __forceinline__ bool reduce_system(double& a, double& b, int tile, co
         r.gpartials[2 * p.gi] = a;
         r.gpartials[2 * p.gi + 1] = b;
         // every group of the system uses its first group's counter
-        last = take_ticket(&r.counters[p.grp0]) == n_groups - 1;
-        if (last) r.counters[p.grp0] = 0;
+        last_group = take_ticket(&r.counters[p.grp0]) == n_groups - 1;
+        if (last_group) r.counters[p.grp0] = 0;
     }
     __syncthreads();
-    if (!last) return false;
+    if (!last_group) return false;
     sum_pairs(r.gpartials, p.grp0, p.grp1, a, b);
     return true;
 }

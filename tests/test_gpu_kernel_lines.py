@@ -294,3 +294,35 @@ def test_setup_with_repeated_columns(gpu, n, per_row):
     h = cb.AmgHierarchy(view, s)
     for _ in range(2):
         _same_hierarchies(cb.AmgHierarchy(view, s, device=True), h)
+
+
+@pytest.mark.parametrize("tiles", [1, 32, 33, 444, 0])
+def test_each_norm_of_the_ldu_solve_over_any_number_of_tiles(gpu, tiles):
+    """The three norms over one tile to more than one group (0: 2050 tiles, the second group of two),
+    from a random x. Residual and reference norm are sums of positive terms (n EPS between two
+    orders); the squared norm sets the target of the solve, which then takes the oracle's iterations
+    (within 2, the order of BiCGStab's sums) and ends at the target. Every repetition is the same."""
+    cb = gpu
+    n = 2049 * 256 + 1
+    own, nei, up, lo, diag, src = _banded(n, 1)
+    diag = diag + 1.0
+    ds = cb.DeviceSolver(cb.build_csr_pattern(n, own, nei))
+    ds.set_tuning(cb.Tuning(target_tiles=tiles))
+    a = _csr(n, own, nei, diag, up, lo)
+    x0 = np.random.default_rng(6).standard_normal(n)
+    want = O.normalised_residual(own, nei, diag, up, lo, src, x0)
+    r0 = np.linalg.norm(src - a.matvec(x0))
+    rel = 1e-7
+    xo, so = O.krylov(a, src, x0, method=1, abs_tol=rel * r0, max_iterations=500)
+    s = cb.LduSettings(method=cb.Method.BiCgStab, tolerance=1e-14, rel_tolerance=rel)
+    first = None
+    for _ in range(4):
+        x = x0.copy()
+        r = ds.solve_ldu(diag, up, lo, src, x, s)
+        assert abs(r.initial_residual - want) <= n * EPS * want
+        assert abs(r.iterations - so["iterations"]) <= 2
+        assert np.linalg.norm(src - a.matvec(x)) <= 1.05 * rel * r0
+        if first is None:
+            first = (r.initial_residual, r.final_residual, r.iterations, x)
+        assert (r.initial_residual, r.final_residual, r.iterations) == first[:3] and np.array_equal(x, first[3])
+    ds.close()
