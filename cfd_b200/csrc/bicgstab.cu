@@ -322,7 +322,7 @@ SolveResult Engine::solve_bicgstab(const SolveRequest& rq, bool want_true) {
     CFDB_CUDA(cudaMemcpyAsync(bcg_st_, &h->s, sizeof(BcgState), cudaMemcpyHostToDevice, stream_));
     CFDB_CUDA(cudaMemcpyAsync(n_active_, h->words, 2 * sizeof(int), cudaMemcpyHostToDevice, stream_));
     launch_graph(kBcgGraphs, kInit);
-    iterate(kBcgGraphs, std::max(rq.max_it, 0) + 1);
+    iterate(kBcgGraphs, std::max(rq.max_it, 0) + 1LL);
     h->cg.true_res = -1.0;
     if (want_true) {
         // |b - A x| of the returned solution, as the CG paths report it

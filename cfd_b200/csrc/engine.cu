@@ -1759,8 +1759,8 @@ Progress Engine::wait_progress(int seq) {
     return r;
 }
 
-void Engine::iterate(int row, int cap) {
-    for (int k = 0; k < cap; ++k) {
+void Engine::iterate(int row, long long cap) {
+    for (long long k = 0; k < cap; ++k) {
         launch_graph(row, kIterate);
         ++published_;
         if (k == 0) continue; // one iteration stays in flight ahead of the records
@@ -1820,8 +1820,9 @@ std::vector<SolveResult> Engine::solve(Mode mode, const std::vector<SolveRequest
         CFDB_CUDA(cudaMemcpyAsync(hs, st_, st_bytes, cudaMemcpyDeviceToHost, stream_));
         CFDB_CUDA(cudaStreamSynchronize(stream_));
     };
-    for (int round = 0; round <= max_it; ++round) {
-        iterate(row, max_it + 2);
+    // (64-bit counts: max_it may be the largest int)
+    for (long long round = 0; round <= max_it; ++round) {
+        iterate(row, max_it + 2LL);
         if (mode == Mode::AmgMixed) launch_graph(row, kVerify);
         else if (want_true) true_residuals();
         read_states();

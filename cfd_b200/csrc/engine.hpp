@@ -254,7 +254,7 @@ private:
     void capture(int row, GraphPiece piece, const std::function<void()>& enqueue);
     void launch_graph(int row, GraphPiece piece);
     // launches iterations until no system is active, an error is flagged or `cap` are launched
-    void iterate(int row, int cap);
+    void iterate(int row, long long cap);
     Progress wait_progress(int seq);
     [[noreturn]] void fail_wait(int error);
     void mark(const char* name, int level, double bytes);

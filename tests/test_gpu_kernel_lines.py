@@ -326,3 +326,29 @@ def test_each_norm_of_the_ldu_solve_over_any_number_of_tiles(gpu, tiles):
             first = (r.initial_residual, r.final_residual, r.iterations, x)
         assert (r.initial_residual, r.final_residual, r.iterations) == first[:3] and np.array_equal(x, first[3])
     ds.close()
+
+
+@pytest.mark.parametrize("limit", [2 ** 31 - 2, 2 ** 31 - 1])
+def test_largest_iteration_limits(gpu, limit):
+    """A limit at the end of the int range is no limit: every method takes the iterations it takes
+    under a limit of 1000."""
+    cb = gpu
+    case = W.cavity(8)
+    up, lo, diag, src = _pressure(case)
+    tol = 1e-8 * np.linalg.norm(src)
+    ds = cb.DeviceSolver(cb.build_csr_pattern(case.n, case.owner, case.neighbour))
+    for method, amg, precision in ((cb.Method.BiCgStab, False, cb.Precision.FP64),
+                                   (cb.Method.Cg, False, cb.Precision.FP64),
+                                   (cb.Method.Cg, True, cb.Precision.FP64),
+                                   (cb.Method.Cg, True, cb.Precision.MIXED)):
+        ds.set_precision(precision)
+        if amg:
+            ds.setup_amg(diag, up, lo, cb.AmgSettings(strength_threshold=0.04, coarse_size=50))
+        got = []
+        for m in (1000, limit):
+            x = np.zeros(case.n)
+            st = ds.solve(diag, up, lo, src, x, method, amg, cb.SolveControl(tol, m))
+            assert st.converged
+            got.append((st.iterations, x))
+        assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])
+    ds.close()
