@@ -878,8 +878,8 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
         red_.gcounters = cnt + n_groups;
         red_.sys_tile0 = arena_.upload(sys_tile0, st);
         red_.grp0 = arena_.upload(grp0, st);
-        seq_ = arena_.alloc<int>(1);
-        CFDB_CUDA(cudaMemsetAsync(seq_, 0, sizeof(int), st));
+        seq_ = arena_.alloc<unsigned>(1);
+        CFDB_CUDA(cudaMemsetAsync(seq_, 0, sizeof(unsigned), st));
         progress_->seq = 0;
         published_ = 0;
         tail_bar_ = arena_.alloc<unsigned>(2);
@@ -1739,13 +1739,13 @@ void Engine::launch_graph(int row, GraphPiece piece) {
 
 // The record `seq` (or a later one). The stream is looked at now and then, so that a failed launch
 // or kernel ends the wait with its error.
-Progress Engine::wait_progress(int seq) {
+Progress Engine::wait_progress(unsigned seq) {
     const volatile Progress* p = progress_;
-    for (unsigned spin = 0; p->seq < seq; ++spin) {
+    for (unsigned spin = 0; !record_reached(p->seq, seq); ++spin) {
         if (spin % 4096 != 4095) continue;
         const cudaError_t e = cudaStreamQuery(stream_);
         if (e == cudaSuccess) {
-            if (p->seq < seq) fail(7, "solve: the stream is idle before its iterations were published");
+            if (!record_reached(p->seq, seq)) fail(7, "solve: the stream is idle before its iterations were published");
         } else if (e != cudaErrorNotReady) {
             CFDB_CUDA(e);
         }

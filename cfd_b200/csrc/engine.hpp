@@ -13,6 +13,7 @@
 #include "host_algos.hpp"
 #include "kernels.cuh"
 #include "ldu_solve.hpp"
+#include "progress_rule.hpp"
 
 namespace cfdb {
 
@@ -255,7 +256,7 @@ private:
     void launch_graph(int row, GraphPiece piece);
     // launches iterations until no system is active, an error is flagged or `cap` are launched
     void iterate(int row, long long cap);
-    Progress wait_progress(int seq);
+    Progress wait_progress(unsigned seq);
     [[noreturn]] void fail_wait(int error);
     void mark(const char* name, int level, double bytes);
     void release_graphs();
@@ -304,7 +305,7 @@ private:
     Reduce red_{};
     int* n_active_ = nullptr; // behind the systems' states: one upload starts a solve
     int* error_ = nullptr;
-    int* seq_ = nullptr;           // device count of published records
+    unsigned* seq_ = nullptr;      // device count of published records
     // Page-locked, mapped: the last record, and behind it the image of the states and the two words
     // behind them (host_state; h_state_ where many systems need more). One small block made with the
     // engine: page-locking a megabyte costs milliseconds, which a first solve should not pay (a new
@@ -312,7 +313,7 @@ private:
     static constexpr size_t kHostBlock = 16 << 10;
     Progress* progress_ = nullptr;
     void* host_state(size_t bytes);
-    int published_ = 0;            // records published by the work launched so far
+    unsigned published_ = 0;       // records published by the work launched so far
     PinnedBuffer h_state_;
     // coarse blocks
     int n_blocks_ = 0;

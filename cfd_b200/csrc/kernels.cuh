@@ -110,7 +110,7 @@ struct Control {
 struct Progress {
     int n_active;
     int error;
-    int seq; // records published so far (written last)
+    unsigned seq; // number of the record (written last; progress_rule.hpp)
 };
 
 // Polls allowed to drain a CTA's own bulk copy after its bounded wait expired: the CTA must
@@ -1421,9 +1421,9 @@ static __global__ void __launch_bounds__(kBlock, (kMinBlocks<double, V, false>))
 }
 
 // The record of one iteration for the host (one thread; the last kernel of its graph).
-static __global__ void k_publish(const int* n_active, const int* error, int* seq, Progress* host) {
+static __global__ void k_publish(const int* n_active, const int* error, unsigned* seq, Progress* host) {
     pdl_entry();
-    const int k = *seq + 1;
+    const unsigned k = *seq + 1;
     *seq = k;
     volatile Progress* h = host;
     h->n_active = *n_active;
