@@ -47,6 +47,7 @@ namespace {
 
 constexpr int kEmpty = INT_MAX; // free table slot; sorts after every column index
 constexpr int kErrInternal = 7; // CFDB_ERR_INTERNAL
+constexpr int kErrOutOfMemory = 3; // CFDB_ERR_OOM
 constexpr int kThreads = 256;
 
 template <int G> __device__ __forceinline__ void group_sync() {
@@ -108,7 +109,8 @@ __device__ long long block_exclusive_scan(long long v, long long* sh, long long*
 __global__ void __launch_bounds__(kScanThreads) k_scan_sums(const int* __restrict__ in, int n, long long* bsum) {
     __shared__ long long sh[32];
     const long long i0 = static_cast<long long>(blockIdx.x) * kScanChunk + 2 * threadIdx.x;
-    const long long v = (i0 < n ? in[i0] : 0) + (i0 + 1 < n ? in[i0 + 1] : 0);
+    const long long v0 = i0 < n ? in[i0] : 0, v1 = i0 + 1 < n ? in[i0 + 1] : 0;
+    const long long v = v0 + v1;
     long long total = 0;
     block_exclusive_scan(v, sh, &total);
     if (threadIdx.x == 0) bsum[blockIdx.x] = total;
@@ -302,14 +304,45 @@ constexpr int kSeedBatch = 4;   // sweeps per host check
 constexpr int kSeedPolls = 128; // looks of a row per sweep
 constexpr int kSeedLook = 8;    // conflicts looked at together
 
+// Entries of the conflict lists per strong entry up to which a level is aggregated on the device. A
+// regular graph of d strong entries a row has about (d + 1) / 2: 2 to 6 on the levels of box, graded and
+// tet meshes, 16 at 29 a row. What lies above 24 (96 bytes per strong entry) are graphs with hubs, columns that
+// many rows are strongly connected to: a hub of m rows alone gives m^2 / 2, each found by a walk along
+// its column, where the host's pass takes m steps.
+constexpr int kConflictsPerStrong = 24;
+
+// *bound += an upper bound of the conflict lists' length: every pair of occurrences in a column and its own row
+__global__ void __launch_bounds__(kThreads) k_conflict_bound(int n, const int* __restrict__ trp, unsigned long long* bound) {
+    __shared__ unsigned long long sh[kThreads / 32];
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long v = 0;
+    if (j < n) {
+        const unsigned long long m = static_cast<unsigned long long>(trp[j + 1] - trp[j]) + 1;
+        v = m * (m - 1) / 2;
+    }
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kThreads / 32; ++w) v += sh[w];
+        if (v != 0) atomicAdd(bound, v);
+    }
+}
+
 // The earlier conflicts of every row (FILL = false: their number): for each j in N[i], the rows s < i
-// with j in N[s]. A row may be listed more than once.
+// with j in N[s]. A row may be listed more than once. FILL = false with *bound above `limit`: counts whose
+// sum is above INT_MAX (n > 1), so that the caller's read of the sum tells it, and no walk.
 template <bool FILL>
 __global__ void k_conflicts(int n, const int* __restrict__ srp, const int* __restrict__ sci,
                             const int* __restrict__ trp, const int* __restrict__ tci, int* cnt,
-                            const int* __restrict__ crp, int* cci) {
+                            const int* __restrict__ crp, int* cci, const unsigned long long* bound,
+                            unsigned long long limit) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (!FILL && *bound > limit) {
+        cnt[i] = i < 2 ? INT_MAX : 0;
+        return;
+    }
     int c = FILL ? crp[i] : 0;
     const int k0 = srp[i], k1 = srp[i + 1];
     if (k1 > k0) { // a row without strong connections is no seed: it needs none
@@ -1431,13 +1464,18 @@ bool device_aggregation(int n, long long ns) { return n >= 4096 && ns <= 20LL * 
 // The aggregation on the device from the strength graph (srp, sci, sav = |a_ij|): passes 1 and
 // 2 in parallel, pass 3 by one thread when at most kPass3Device rows are left for it. agg
 // receives every row's aggregate. Returns the number of aggregates, or -1 when more rows are
-// left for pass 3 (isolated rows, or rows none of whose strong neighbours pass 1 aggregated), or the
-// conflict lists pass 2^31 entries: the caller then aggregates on the host.
+// left for pass 3 (isolated rows, or rows none of whose strong neighbours pass 1 aggregated), when the
+// conflict lists pass kConflictsPerStrong or 2^31 entries, or when there is no memory for them: the
+// caller then aggregates on the host.
 int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, int* agg) {
     cudaStream_t st = cx.st;
-    // scratch of its own (the transpose, conflict lists), given back before the products need theirs;
-    // every path out of here has synchronised st
+    // scratch of its own (the transpose, conflict lists), given back before the products need theirs and
+    // after st's work on it
     Scratch own;
+    struct Drain {
+        cudaStream_t st;
+        ~Drain() { cudaStreamSynchronize(st); }
+    } drain{st};
     Ctx tx = cx;
     tx.mem = &own;
     tx.keep = nullptr;
@@ -1453,11 +1491,15 @@ int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, in
     k_seed_init<<<grid_for(n), kThreads, 0, st>>>(n, srp, state);
     int* ccnt = tx.mem->alloc<int>(static_cast<size_t>(n) + 1);
     int* crp = tx.mem->alloc<int>(static_cast<size_t>(n) + 1);
-    k_conflicts<false><<<grid_for(n), kThreads, 0, st>>>(n, srp, sci, t.rp, t.ci, ccnt, nullptr, nullptr);
+    auto* bound = tx.mem->alloc<unsigned long long>(1);
+    CFDB_CUDA(cudaMemsetAsync(bound, 0, sizeof(*bound), st));
+    k_conflict_bound<<<grid_for(n), kThreads, 0, st>>>(n, t.rp, bound);
+    const unsigned long long limit = static_cast<unsigned long long>(kConflictsPerStrong) * static_cast<unsigned>(ns);
+    k_conflicts<false><<<grid_for(n), kThreads, 0, st>>>(n, srp, sci, t.rp, t.ci, ccnt, nullptr, nullptr, bound, limit);
     const long long n_conf = scan(tx, ccnt, n, crp);
     if (n_conf > INT_MAX) return -1;
     int* cci = tx.mem->alloc<int>(static_cast<size_t>(n_conf));
-    k_conflicts<true><<<grid_for(n), kThreads, 0, st>>>(n, srp, sci, t.rp, t.ci, nullptr, crp, cci);
+    k_conflicts<true><<<grid_for(n), kThreads, 0, st>>>(n, srp, sci, t.rp, t.ci, nullptr, crp, cci, nullptr, 0);
     int* at = ccnt; // conflicts passed so far
     CFDB_CUDA(cudaMemsetAsync(at, 0, sizeof(int) * static_cast<size_t>(n), st));
     // lo of each sweep of a batch; lo[0] = 0, then the last lo of the previous batch
@@ -1465,8 +1507,8 @@ int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, in
     CFDB_CUDA(cudaMemsetAsync(lo, 0, sizeof(int), st));
     const int grid = grid_for(std::min(n, kSeedWindow));
     for (long long sweeps = 0;;) {
-        // every sweep decides at least its smallest undecided row
-        if (sweeps > n + kSeedBatch) fail(kErrInternal, "device aggregation did not settle");
+        // in every sweep its smallest undecided row is decided, or passes kSeedPolls x kSeedLook of its conflicts
+        if (sweeps > n + n_conf / (kSeedPolls * kSeedLook) + kSeedBatch) fail(kErrInternal, "device aggregation did not settle");
         CFDB_CUDA(cudaMemsetAsync(lo + 1, 0x7f, sizeof(int) * kSeedBatch, st));
         for (int b = 0; b < kSeedBatch; ++b)
             k_seed_sweep<<<grid, kThreads, 0, st>>>(n, lo + b, lo + b + 1, crp, cci, at, state);
@@ -1581,11 +1623,18 @@ void amg_setup_device(const DevCsr& a0, const AmgSettings& s, cudaStream_t st, D
         });
         CFDB_CUDA(cudaGetLastError());
         phase("strength");
-        // aggregation: passes 1 and 2 on the device; when rows are left for pass 3 the host runs
-        // all three passes from the strength graph
+        // aggregation on the device; on the host, all three passes from the strength graph, for the
+        // levels that device_aggregation or aggregate_device refuse
         std::vector<int> agg;
         int* dagg = h.mem.alloc<int>(nl);
-        int n_agg = device_aggregation(nl, ns) ? aggregate_device(cx, nl, ns, srp, sci, sav, dagg) : -1;
+        int n_agg = -1;
+        if (device_aggregation(nl, ns)) {
+            try {
+                n_agg = aggregate_device(cx, nl, ns, srp, sci, sav, dagg);
+            } catch (const Error& e) {
+                if (e.code != kErrOutOfMemory) throw;
+            }
+        }
         if (n_agg < 0) {
             // read back: offsets, columns and, per entry, its strength rank within the row (2
             // bytes; the |a_ij| themselves when a row has more than 65536 strong entries)

@@ -352,3 +352,36 @@ def test_largest_iteration_limits(gpu, limit):
             got.append((st.iterations, x))
         assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])
     ds.close()
+
+
+def _with_hub(n, half, degree, seed=9):
+    """_banded with row n // 2 connected to `degree` further rows."""
+    own, nei, up, lo, diag, _ = _banded(n, half, seed)
+    hub = n // 2
+    far = np.setdiff1d(np.arange(n), np.arange(hub - half, hub + half + 1))
+    far = np.sort(np.random.default_rng(seed).permutation(far)[:degree])
+    w = np.random.default_rng(seed + 1).uniform(0.5, 1.5, degree)
+    diag = diag.copy()
+    np.add.at(diag, far, w)
+    diag[hub] += w.sum()
+    own = np.concatenate([own, np.minimum(far, hub).astype(np.int32)])
+    nei = np.concatenate([nei, np.maximum(far, hub).astype(np.int32)])
+    o = np.lexsort((nei, own))
+    v = np.concatenate([up, -w])[o]
+    return _csr(n, own[o], nei[o], diag, v, v.copy())
+
+
+@pytest.mark.parametrize("n,degree", [(9000, 300), (9000, 1200), (9000, 1400), (9000, 8900), (60000, 59000)])
+def test_setup_with_a_hub_row(gpu, n, degree):
+    """One row strongly connected to many: its rows conflict pairwise (degree^2 / 2), which the device
+    aggregates up to 24 conflicts a strong entry (degrees to about 1300 of 9000 rows) and the host beyond.
+    Equal to the host build, within memory in proportion to the matrix."""
+    import torch
+    cb = gpu
+    a = _with_hub(n, 2, degree)
+    view = cb.CsrView(a.n_rows, a.rp, a.ci, a.va)
+    s = cb.AmgSettings(strength_threshold=0.0, max_levels=2)
+    h = cb.AmgHierarchy(view, s)
+    free = torch.cuda.mem_get_info()[0]
+    _same_hierarchies(cb.AmgHierarchy(view, s, device=True), h)
+    assert free - torch.cuda.mem_get_info()[0] <= (256 << 20) + 1000 * a.va.nbytes
