@@ -2,7 +2,8 @@
 
 The knobs are those of `Tuning` (include/cfdb.h, cfdb_tuning):
 
-* target_tiles - level-0 Krylov tiles (0: 256 rows each; else at most about this many CTAs),
+* target_tiles - level-0 Krylov tiles (0: 256 rows each; else at most about this many CTAs, up to
+                 the default as few as tiles of 4096 rows allow),
 * wide_row     - average row length above which a level switches from SELL-32 rows to
                  CSR lane groups,
 * lanes_div    - lanes per CSR row = 4 x average row length / lanes_div,

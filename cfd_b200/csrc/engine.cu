@@ -345,11 +345,13 @@ int csr_lanes(double rows, double avg, int lanes_div, bool fp64) {
 // waves of 7-entry rows, or one and a few CTAs) against this rule: graded 885K cells FP64 5.22
 // against 4.95 ms, 176K cells mixed 1.29 against 1.19, scalar step (BiCGStab, 512K cells) 1.15
 // against 0.98, 304K tets mixed 1.81 against 1.73. 5.1M tets (8690 rows a tile in one wave): 11.63
-// ms in one wave, 11.35 in two, 11.53 in three.
+// ms in one wave, 11.35 in two, 11.53 in three (the one mesh beyond 4096 rows a tile). A target
+// above the default asks for shorter tiles: as many whole waves as it holds.
 int krylov_tiles(int rows, int visit, int target) {
     const int wave = 148 * krylov_ctas(visit);
     if (target <= wave) return target;
-    return wave * std::min(target / wave, ceil_div(rows, 4096 * wave));
+    const int waves = target / wave;
+    return wave * (target > Tuning{}.target_tiles ? waves : std::min(waves, ceil_div(rows, 4096 * wave)));
 }
 
 int grid_of(long long n) { return static_cast<int>(std::max<long long>(1, (n + 255) / 256)); }

@@ -41,7 +41,8 @@ struct SystemSpec {
 // Launch-shape and schedule knobs (no effect on the arithmetic of a row sum except that wide
 // operators switch between the ordered SELL sum and the lane-group CSR sum).
 struct Tuning {
-    int target_tiles = 148 * 8; // level-0 Krylov tiles: at most about this many (0: 256 rows each)
+    int target_tiles = 148 * 8; // level-0 Krylov tiles: at most about this many (0: 256 rows each); up to
+                                // this default fewer on smaller systems (krylov_tiles)
     int wide_row = 48;          // average row length above which CSR lane groups are used
     int lanes_div = 16;         // lanes per CSR row ~ 4 x average row length / lanes_div (4..256),
                                 // within a wave of threads per operator

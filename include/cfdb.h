@@ -424,8 +424,8 @@ int cfdb_system_kernel_launches(const cfdb_system* sys, unsigned long long* coun
 /* Launch-shape / schedule knobs of the device plan (see cfd_b200/autotune.py). */
 typedef struct {
     int target_tiles; /* level-0 Krylov tiles (reductions): at most about this many CTAs (whole
-                         waves of resident ones, as few as tiles of 4096 rows allow), default 1184 =
-                         148 SMs x 8; 0 = 256 rows per CTA */
+                         waves of resident ones; up to the default as few as tiles of 4096 rows
+                         allow), default 1184 = 148 SMs x 8; 0 = 256 rows per CTA */
     int wide_row;     /* average row length above which CSR lane groups are used, default 48 */
     int lanes_div;    /* lanes per CSR row ~ 4 x average row length / lanes_div (4..256, within about a
                          wave of threads per operator), default 16 */

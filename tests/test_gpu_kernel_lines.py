@@ -385,3 +385,25 @@ def test_setup_with_a_hub_row(gpu, n, degree):
     free = torch.cuda.mem_get_info()[0]
     _same_hierarchies(cb.AmgHierarchy(view, s, device=True), h)
     assert free - torch.cuda.mem_get_info()[0] <= (256 << 20) + 1000 * a.va.nbytes
+
+
+def _cg(cb, ds, diag, up, lo, src, tiles, method=0, pair=1):
+    """Solution of a Jacobi-preconditioned solve; its bits depend on how the sums are cut into tiles."""
+    ds.set_tuning(cb.Tuning(target_tiles=tiles, krylov_pair=pair))
+    x = np.zeros(len(diag))
+    ds.solve(diag, up, lo, src, x, method, False, cb.SolveControl(1e-10 * np.linalg.norm(src), 500))
+    return x
+
+
+def test_target_above_the_default_gives_shorter_tiles(gpu):
+    """524545 rows of 3 entries: the default takes one wave of CTAs, 2368 four waves, which is tiles of
+    256 rows here, as 0 asks for."""
+    cb = gpu
+    n = 2049 * 256 + 1
+    own, nei, up, lo, diag, src = _banded(n, 1)
+    diag = diag + 1.0
+    ds = cb.DeviceSolver(cb.build_csr_pattern(n, own, nei))
+    x = {t: _cg(cb, ds, diag, up, lo, src, t) for t in (0, 592, 148 * 8, 148 * 16)}
+    assert np.array_equal(x[148 * 16], x[0])
+    assert np.array_equal(x[148 * 8], x[592]) and not np.array_equal(x[592], x[0])
+    ds.close()
