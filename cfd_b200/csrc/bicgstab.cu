@@ -260,12 +260,6 @@ static __global__ void __launch_bounds__(kBlock) k_bcg_xr(Tiles tiles, BcgState*
 
 } // namespace
 
-// fn with the stream strategy of the level-0 operator.
-template <class Fn> void Engine::with_krylov(Fn&& fn) const {
-    if (krylov_visit_of(row_width(lv_[0].a), true) == kVisitStream5) fn(std::integral_constant<int, kVisitStream5>{});
-    else fn(std::integral_constant<int, kVisitStream7>{});
-}
-
 // The initial residual, or the five kernels of one iteration.
 void Engine::enqueue_bicgstab(bool init) {
     const DevLevel& d = lv_[0];
@@ -290,7 +284,7 @@ void Engine::enqueue_bicgstab(bool init) {
         launch_k(pdl, k_bcg_spmv<kV, true>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles, bcg_st_, sh, s, t, red_, n_active_);
         launch_k(pdl, k_bcg_xr, d.n_tiles, kBlock, 0, stream_, d.tiles, bcg_st_, ph, sh, s, t, r0, x_, r_, red_, n_active_);
     };
-    with_krylov(run);
+    with_krylov_visit(krylov_visit(), run);
 }
 
 SolveResult Engine::solve_bicgstab(const SolveRequest& rq, bool want_true) {
@@ -326,7 +320,7 @@ SolveResult Engine::solve_bicgstab(const SolveRequest& rq, bool want_true) {
     h->cg.true_res = -1.0;
     if (want_true) {
         // |b - A x| of the returned solution, as the CG paths report it
-        with_krylov([&](auto V) {
+        with_krylov_visit(krylov_visit(), [&](auto V) {
             launch_k(tuning_.pdl != 0, k_true_residual<decltype(V)::value>, d.n_tiles, kBlock, 0, stream_, d.a.s64, d.tiles,
                      st_, b_, x_, red_);
         });

@@ -501,38 +501,6 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
     off0_.resize(n_sys_);
     for (int s = 0; s < n_sys_; ++s) off0_[s] = off[0][s];
     cudaStream_t st = stream_;
-    // Krylov tiles of level 0 (the reductions): kSellRows rows, or a tile count when target_tiles > 0;
-    // coarser levels use their operators' own tiles
-    std::vector<int> sys_tile0(n_sys_ + 1, 0);
-    double nnz0 = 0.0;
-    for (const SystemSpec& sp : systems) nnz0 += sp.rp[sp.n];
-    for (int l = 0; l < 1; ++l) {
-        DevLevel& d = lv_[l];
-        const int rows0 = std::max(d.n_rows, 1);
-        const int visit0 = krylov_visit_of(nnz0 / rows0, tuning_.krylov_pair != 0);
-        const int base = tuning_.target_tiles > 0
-                             ? std::max(kSellRows, round_up(ceil_div(rows0, krylov_tiles(rows0, visit0, tuning_.target_tiles)), kSellRows))
-                             : kSellRows;
-        std::vector<int> trow, tsys;
-        int nc_tiles = -1;
-        for (int k = 0; k < n_sys_; ++k) {
-            const int s = perm_[k];
-            if (L[s] <= l) continue;
-            if (L[s] - 1 == l && nc_tiles < 0) nc_tiles = static_cast<int>(tsys.size());
-            if (l == 0) sys_tile0[k] = static_cast<int>(tsys.size());
-            const int pad = round_up(rows_at(s, l), 32);
-            for (int r = 0; r < pad; r += base) {
-                trow.push_back(off[l][s] + r);
-                tsys.push_back(k);
-            }
-        }
-        if (l == 0) sys_tile0[n_sys_] = static_cast<int>(tsys.size());
-        trow.push_back(d.n_rows);
-        d.n_tiles = static_cast<int>(tsys.size());
-        d.n_tiles_nc = nc_tiles < 0 ? d.n_tiles : nc_tiles;
-        d.tiles.row = arena_.upload(trow, st);
-        d.tiles.sys = n_sys_ > 1 ? arena_.upload(tsys, st) : nullptr;
-    }
     // Launch tiles of one operator over the rows of `row_level` of the systems `include`
     // selects (a prefix in batch order); `nc` marks the systems that continue past that level.
     auto op_tiles = [&](DevSell64_32& m, int fmt, int row_level, auto include, auto nc) {
@@ -674,6 +642,37 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
             l0_ = L0Cache{d.a, d.wd64, d.wd32, src0_, diag_src0_, row_map_, dinv0_, user_rows_};
             l0_valid_ = true;
         }
+    }
+    // Krylov tiles of level 0 (the reductions), sized for the kernels that krylov_visit() picks for its
+    // operator: kSellRows rows, or a tile count when target_tiles > 0, cut per system and rounded up to
+    // kSellRows rows (a batch, or a system of few rows a tile, then leaves its last wave part empty);
+    // coarser levels use their operators' own tiles
+    std::vector<int> sys_tile0(n_sys_ + 1, 0);
+    {
+        DevLevel& d = lv_[0];
+        const int rows0 = std::max(d.n_rows, 1);
+        const int base =
+            tuning_.target_tiles > 0
+                ? std::max(kSellRows, round_up(ceil_div(rows0, krylov_tiles(rows0, krylov_visit(), tuning_.target_tiles)), kSellRows))
+                : kSellRows;
+        std::vector<int> trow, tsys;
+        int nc_tiles = -1;
+        for (int k = 0; k < n_sys_; ++k) {
+            const int s = perm_[k];
+            if (L[s] == 1 && nc_tiles < 0) nc_tiles = static_cast<int>(tsys.size());
+            sys_tile0[k] = static_cast<int>(tsys.size());
+            const int pad = round_up(rows_at(s, 0), 32);
+            for (int r = 0; r < pad; r += base) {
+                trow.push_back(off[0][s] + r);
+                tsys.push_back(k);
+            }
+        }
+        sys_tile0[n_sys_] = static_cast<int>(tsys.size());
+        trow.push_back(d.n_rows);
+        d.n_tiles = static_cast<int>(tsys.size());
+        d.n_tiles_nc = nc_tiles < 0 ? d.n_tiles : nc_tiles;
+        d.tiles.row = arena_.upload(trow, st);
+        d.tiles.sys = n_sys_ > 1 ? arena_.upload(tsys, st) : nullptr;
     }
     phase("plan_level0");
     // coarser levels, transfers
@@ -1107,16 +1106,6 @@ template <class Fn> void with_visit(int v, Fn&& fn) {
     case kVisitStream7: fn(std::integral_constant<int, kVisitStream7>{}); break;
     case kVisitWarp: fn(std::integral_constant<int, kVisitWarp>{}); break;
     default: fn(std::integral_constant<int, kVisitBlock>{}); break;
-    }
-}
-
-// The strategies of krylov_visit_of.
-template <class Fn> void with_krylov_visit(int v, Fn&& fn) {
-    switch (v) {
-    case kVisitSell5: fn(std::integral_constant<int, kVisitSell5>{}); break;
-    case kVisitSell7: fn(std::integral_constant<int, kVisitSell7>{}); break;
-    case kVisitStream5: fn(std::integral_constant<int, kVisitStream5>{}); break;
-    default: fn(std::integral_constant<int, kVisitStream7>{}); break;
     }
 }
 } // namespace

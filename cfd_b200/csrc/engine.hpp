@@ -298,7 +298,6 @@ private:
     NormState* norms_ = nullptr; // residual_norms (allocated on first use)
     Reduce red2_{};
     void enqueue_bicgstab(bool init);
-    template <class Fn> void with_krylov(Fn&& fn) const;
     // Krylov vectors (level 0)
     double *b_ = nullptr, *x_ = nullptr, *r_ = nullptr, *p_ = nullptr, *q_ = nullptr;
     // state

@@ -20,6 +20,7 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <type_traits>
 
 namespace cfdb {
 
@@ -632,6 +633,16 @@ __host__ __device__ inline int visit_of(int fmt, double width, int tiles, bool f
 __host__ __device__ inline int krylov_visit_of(double width, bool ahead) {
     if (width <= 5.25) return ahead ? kVisitStream5 : kVisitSell5;
     return ahead ? kVisitStream7 : kVisitSell7;
+}
+
+// Calls fn with a strategy of krylov_visit_of as a compile-time constant.
+template <class Fn> void with_krylov_visit(int v, Fn&& fn) {
+    switch (v) {
+    case kVisitSell5: fn(std::integral_constant<int, kVisitSell5>{}); break;
+    case kVisitSell7: fn(std::integral_constant<int, kVisitSell7>{}); break;
+    case kVisitStream5: fn(std::integral_constant<int, kVisitStream5>{}); break;
+    default: fn(std::integral_constant<int, kVisitStream7>{}); break;
+    }
 }
 
 // CTAs per SM of the level-0 Krylov kernels.

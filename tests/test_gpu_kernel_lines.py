@@ -407,3 +407,30 @@ def test_target_above_the_default_gives_shorter_tiles(gpu):
     assert np.array_equal(x[148 * 16], x[0])
     assert np.array_equal(x[148 * 8], x[592]) and not np.array_equal(x[592], x[0])
     ds.close()
+
+
+@pytest.mark.parametrize("method", [0, 1])
+def test_tiles_are_planned_for_the_kernels_that_run(gpu, method):
+    """300000 rows of 3 entries, every 16th of 9: its slices are 9 wide, so the kernels for 7 entries a
+    row run, with 3 CTAs per SM loading ahead and 6 one row at a time. The default tiles are one wave of
+    those (444 and 888); BiCGStab (method 1) takes rows as CG does, with the same bits either way."""
+    cb = gpu
+    n = 300000
+    own, nei, up, lo, diag, src = _banded(n, 1)
+    hub = np.arange(8, n - 8, 16)
+    far = np.concatenate([np.stack([np.minimum(hub, hub + k), np.maximum(hub, hub + k)], 1) for k in (-7, -5, -3, 2, 4, 6)])
+    pairs = np.concatenate([np.stack([own, nei], 1), far])
+    w = np.concatenate([-up, np.full(len(far), 0.25)])
+    o = np.lexsort((pairs[:, 1], pairs[:, 0]))
+    pairs, w = pairs[o].astype(np.int32), w[o]
+    own, nei = np.ascontiguousarray(pairs[:, 0]), np.ascontiguousarray(pairs[:, 1])
+    diag = np.bincount(own, w, n) + np.bincount(nei, w, n) + 1.0
+    up, lo = -w, -w.copy()
+    ds = cb.DeviceSolver(cb.build_csr_pattern(n, own, nei))
+    a = _csr(n, own, nei, diag, up, lo)
+    assert len(a.va) / n < 5.25
+    x = {(t, p): _cg(cb, ds, diag, up, lo, src, t, method, p) for t in (148 * 8, 444, 888) for p in (0, 1)}
+    assert np.linalg.norm(src - a.matvec(x[444, 1])) <= 1.05e-10 * np.linalg.norm(src)
+    assert np.array_equal(x[148 * 8, 1], x[444, 1]) and np.array_equal(x[148 * 8, 0], x[888, 0])
+    assert np.array_equal(x[444, 0], x[444, 1]) and not np.array_equal(x[888, 0], x[444, 0])
+    ds.close()
