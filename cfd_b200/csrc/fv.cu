@@ -356,6 +356,8 @@ template <class F> int guarded_fv(F&& f) {
 // The launches behind the entry points: arguments checked, work enqueued on the geometry's stream.
 namespace cfdb {
 
+int fv_device(const cfdb_fv* fv) { return fv->device; }
+
 cudaStream_t fv_stream(const cfdb_fv* fv) { return fv->st; }
 
 void fv_gradient(cfdb_fv* fv, const double* p, double* grad, const double* hbya, const double* rau, double* u) {

@@ -9,6 +9,7 @@ struct cfdb_fv;
 
 namespace cfdb {
 
+int fv_device(const cfdb_fv* fv);
 cudaStream_t fv_stream(const cfdb_fv* fv);
 // grad of p; with u also u = hbya - rau grad
 void fv_gradient(cfdb_fv* fv, const double* p, double* grad, const double* hbya, const double* rau, double* u);

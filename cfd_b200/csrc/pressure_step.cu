@@ -75,6 +75,7 @@ extern "C" int cfdb_pressure_correction_device(cfdb_system* sys, cfdb_fv* fv, co
         ok(cfdb_system_stream(sys, &sys_stream), "system stream");
         const cudaStream_t ss = static_cast<cudaStream_t>(sys_stream);
         const cudaStream_t fs = cfdb::fv_stream(fv);
+        CFDB_CUDA(cudaSetDevice(cfdb::fv_device(fv))); // the event belongs to the streams' device
         Order order;
         auto copy = [&](double* dst, const double* src) { CFDB_CUDA(cudaMemcpyAsync(dst, src, bn, cudaMemcpyDeviceToDevice, fs)); };
         auto drain = [&]() {
