@@ -434,3 +434,44 @@ def test_tiles_are_planned_for_the_kernels_that_run(gpu, method):
     assert np.array_equal(x[148 * 8, 1], x[444, 1]) and np.array_equal(x[148 * 8, 0], x[888, 0])
     assert np.array_equal(x[444, 0], x[444, 1]) and not np.array_equal(x[888, 0], x[444, 0])
     ds.close()
+
+
+def test_mixed_batch_with_a_target_out_of_reach(gpu):
+    """Three systems in mixed precision: one whose target lies below the FP64 floor, so that its FP64 check
+    fails and it goes on alone, round after round, and two that reach theirs. Those keep the iterations
+    and the solution that they have without it (the same plan), and every true residual is that of
+    the returned x."""
+    import torch
+    cb = gpu
+    case = W.cavity(12)
+    up, lo, diag, src = _pressure(case)
+    a = _csr(case.n, case.owner, case.neighbour, diag, up, lo)
+    n, k = case.n, 3
+    b = cb.Batch([n] * k, [case.n_faces] * k, np.tile(case.owner[:case.n_faces], k), np.tile(case.neighbour, k))
+    rep = lambda v: np.tile(v, k)  # noqa: E731
+    b.set_precision(cb.Precision.MIXED)
+    b.setup_amg(rep(diag), rep(up), rep(lo), cb.AmgSettings(strength_threshold=0.04, coarse_size=50))
+    T = lambda v: torch.as_tensor(v, dtype=torch.float64, device="cuda")  # noqa: E731
+    rng = np.random.default_rng(2)
+    rhs = np.concatenate([src, rng.standard_normal(n), rng.standard_normal(n)])
+    norm = [np.linalg.norm(rhs[i * n:(i + 1) * n]) for i in range(k)]
+    mag = np.linalg.norm
+    out = {}
+    for far in (1e-8, 1e-18):
+        x = torch.zeros(n * k, dtype=torch.float64, device="cuda")
+        rel = [1e-6, far, 1e-10]
+        st = b.solve_device(T(rep(diag)), T(rep(up)), T(rep(lo)), T(rhs), x,
+                            [cb.SolveControl(r * v, 40) for r, v in zip(rel, norm)])
+        got = x.cpu().numpy()
+        for i in range(k):
+            xi, bi = got[i * n:(i + 1) * n], rhs[i * n:(i + 1) * n]
+            res = mag(bi - a.matvec(xi))
+            assert abs(res - st[i].true_residual) <= 64 * EPS * mag(np.abs(bi) + _abs_matvec(a, xi))
+            assert st[i].converged == (rel[i] > 1e-15) and st[i].iterations <= 40
+            if st[i].converged:
+                assert st[i].true_residual <= rel[i] * norm[i]
+        assert st[1].iterations == 40 or far > 1e-15
+        out[far] = (got, [s.iterations for s in st])
+    for i in (0, 2):
+        assert out[1e-8][1][i] == out[1e-18][1][i]
+        assert np.array_equal(out[1e-8][0][i * n:(i + 1) * n], out[1e-18][0][i * n:(i + 1) * n])

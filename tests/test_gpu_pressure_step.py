@@ -87,3 +87,53 @@ def test_pressure_correction_step_bitwise(gpu, kind, n_corr, majumdar):
     assert np.array_equal(h(p), p_want)
     assert np.array_equal(h(u), O.correct_velocity(want["hbya"], want["rau"], O.pressure_gradient(*grad_args, p_want)))
     fv.close()
+
+
+@pytest.mark.parametrize("n_corr", [2, 3])
+def test_step_on_a_side_stream_with_several_correctors(gpu, n_corr):
+    """The step called on a torch stream of its own, its inputs still being computed there: two library
+    streams ordered by events, several solves of one matrix. Every field equals, bit for bit, that of a
+    call on finished inputs; a second step continues on the first one's results."""
+    import torch
+    cb = gpu
+    from cfd_b200 import pressure as P
+    m, kinds, pout, ufix, mom, u0, u_prev, phi_prev, p0 = _setup(cb, "tet")
+    ni = m.n_internal_faces
+    T = lambda a: torch.as_tensor(np.ascontiguousarray(a), dtype=torch.float64, device="cuda")  # noqa: E731
+    names = ("mom_diag", "mom_upper", "mom_lower", "mom_source")
+    host = [mom[k] for k in names] + [u0, p0, ufix, u_prev, phi_prev]
+    s = P.PressureSettings(alpha_u=0.7, alpha_p=0.3, n_non_orth_correctors=n_corr, ref_cell=-1,
+                           p_solver=cb.LduSettings(tolerance=1e-13, rel_tolerance=1e-6, max_iterations=2000))
+
+    def step(ds, fv, a, phi):
+        init = P.pressure_correction(ds, fv, *a[:6], a[6], s, relax_p=True, u_prev=a[7], phi_prev=a[8], phi=phi)
+        return init
+
+    got = []
+    for side in (False, True):
+        ds = cb.DeviceSolver(mesh=(m.n_cells, m.owner[:ni], m.neighbour))
+        fv = cb.FvGeometry(m, kinds, pout)
+        ready = [T(v) for v in host]
+        phi = torch.zeros(m.n_faces, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        if side:
+            st = torch.cuda.Stream()
+            with torch.cuda.stream(st):
+                busy = torch.ones(4096, 4096, device="cuda")
+                for _ in range(40):
+                    busy = busy @ busy * 1e-4  # milliseconds of work ahead of the inputs
+                wait = 0.0 * torch.nan_to_num(busy[0, 0].double(), 0.0, 0.0, 0.0)
+                a = [torch.empty_like(v).fill_(7.0) for v in ready]
+                for dst, v in zip(a, ready):
+                    dst.copy_(v + wait)
+                init = [step(ds, fv, a, phi), step(ds, fv, a, phi)]
+        else:
+            a = ready
+            init = [step(ds, fv, a, phi), step(ds, fv, a, phi)]
+        torch.cuda.synchronize()
+        got.append(init + [t.cpu().numpy() for t in (a[4], a[5], phi)])
+        fv.close()
+        ds.close()
+    assert got[0][:2] == got[1][:2] and got[0][1] != got[0][0]
+    for x, y in zip(got[0][2:], got[1][2:]):
+        assert np.isfinite(x).all() and np.array_equal(x, y)
