@@ -60,6 +60,12 @@ CANDIDATES = {
 SCHEDULE_KNOBS = (("tail_rows", "tail_cluster"), "sell_rows", "target_tiles", "vcycle_pair")
 
 
+# What the knobs' values mean, kept with a cached result: a result of another meaning is searched
+# again. 2: lanes_div as a quarter of a lane's entries, target_tiles as an upper limit (1, not
+# written: entries per lane, tiles as given).
+KNOBS = 2
+
+
 def _key(t: Tuning) -> tuple:
     return tuple(dataclasses.astuple(t))
 
@@ -125,7 +131,8 @@ def solve_timer(target, run_iterations: Callable[[int], None], stream_handle: in
 def tune(target, run_iterations, stream_handle, signature: str, cache_path: str | None = None,
          iterations: int = 6, reps: int = 3, passes: int = 2):
     """Tunes `target` for the workload named by `signature`, reusing a cached result when the
-    cache file holds one. Installs and returns the best tuning with its record."""
+    cache file holds one of the present knobs (KNOBS). Installs and returns the best tuning with
+    its record."""
     cache = {}
     if cache_path and os.path.exists(cache_path):
         try:
@@ -133,7 +140,7 @@ def tune(target, run_iterations, stream_handle, signature: str, cache_path: str 
                 cache = json.load(f)
         except (OSError, ValueError):
             cache = {}
-    if signature in cache:
+    if cache.get(signature, {}).get("knobs") == KNOBS:
         rec = cache[signature]
         best = Tuning(**rec["tuning"])
         target.set_tuning(best)
@@ -142,7 +149,7 @@ def tune(target, run_iterations, stream_handle, signature: str, cache_path: str 
     default_ms = evaluate(Tuning())
     best, best_ms, trace = coordinate_search(evaluate, Tuning(), passes=passes)
     target.set_tuning(best)
-    rec = {"tuning": dataclasses.asdict(best), "ms": best_ms, "default_ms": default_ms,
+    rec = {"knobs": KNOBS, "tuning": dataclasses.asdict(best), "ms": best_ms, "default_ms": default_ms,
            "iterations": iterations, "evaluations": len(trace), "trace": trace}
     if cache_path:
         cache[signature] = rec

@@ -48,3 +48,35 @@ def test_retune_knobs_keeps_the_schedule_and_searches_only_its_knobs():
     for t in seen:  # every point differs from the base in the schedule knobs alone
         diff = {k for k, v in dataclasses.asdict(t).items() if v != getattr(base, k)}
         assert diff <= names
+
+
+def test_cached_results_of_other_knobs_are_searched_again(tmp_path, monkeypatch):
+    """A cache written under an earlier meaning of the knobs (no version) is replaced, one of the
+    present meaning is read back."""
+    import json
+
+    from cfd_b200 import autotune as A
+
+    class Target:
+        def set_tuning(self, t):
+            self.tuning = t
+
+    calls = []
+
+    def timer(target, run, stream, iterations, reps):
+        def evaluate(t):
+            calls.append(t)
+            return 2.0 - (t.wide_row == 64)
+        return evaluate
+
+    monkeypatch.setattr(A, "solve_timer", timer)
+    path = tmp_path / "cache.json"
+    old = {"tuning": dataclasses.asdict(dataclasses.replace(Tuning(), lanes_div=32)), "ms": 1.0}
+    path.write_text(json.dumps({"mesh": old, "other": old}))
+    target = Target()
+    best, rec = A.tune(target, None, 0, "mesh", str(path))
+    assert not rec["cached"] and calls and best == target.tuning == dataclasses.replace(Tuning(), wide_row=64)
+    n = len(calls)
+    again, rec = A.tune(target, None, 0, "mesh", str(path))
+    assert rec["cached"] and again == best == target.tuning and len(calls) == n
+    assert json.loads(path.read_text())["other"] == old
