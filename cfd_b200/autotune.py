@@ -12,7 +12,8 @@ The knobs are those of `Tuning` (include/cfdb.h, cfdb_tuning):
 * krylov_pair  - level-0 Krylov SpMV kernels load the next row ahead, or take one at a time,
 * krylov_stage - the level-0 Krylov SpMV streams the operator through shared memory by bulk
                  copies in this many buffers (0: the threads load it, as krylov_pair says),
-* tail_rows    - coarse levels of at most this many rows run in one persistent kernel,
+* tail_rows    - coarse levels of at most this many rows run in one persistent kernel, as far up
+                 as their operators are CSR lane groups,
 * vcycle_pair  - V-cycle kernels of SELL operators load the next row ahead, or take one at a time,
 * tail_cluster - that kernel as one thread-block cluster of this many CTAs (0: a cooperative
                  grid), searched jointly with tail_rows (the candidates keep the grid form),

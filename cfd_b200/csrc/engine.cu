@@ -679,9 +679,9 @@ void Engine::build(std::vector<SystemSpec> systems, int sweeps, double weight, b
     for (int l = 0; l < n_levels_; ++l) {
         DevLevel& d = lv_[l];
         // One operator over the systems that continue past level l: rows of each block from
-        // `pick(s)`, columns shifted into the target level's concatenated index space. Wide
-        // operators (more than kWideRow entries per row on average) are stored as CSR for the
-        // warp-per-row kernels unless the engine is in ordered (bit-reproducible) mode.
+        // `pick(s)`, columns shifted into the target level's concatenated index space. Operators
+        // of long or few rows (use_lanes) are stored as CSR for the lane-group kernels unless the
+        // engine is in ordered (bit-reproducible) mode.
         // dsrc: the operator as a device CSR (single-system plans with device-resident levels)
         auto build_op = [&](auto pick, const DevCsr* dsrc, int col_level, int row_level, DevSell64_32& m) {
             long long nnz = 0, rows = 0;
@@ -1348,7 +1348,7 @@ void Engine::enqueue_vcycle_t(bool fused_final, int flexible, bool x1_ready0) {
         const double cb = sizeof(T) == 4 && m.s32.c16 != nullptr ? 2.0 : 4.0;
         return static_cast<double>(m.nnz) * (sv + cb) + 4.0 * (rows + 1.0) + sv * cols + sv * rows;
     };
-    // tiles of an operator: one row per warp for CSR operators, slice runs for SELL ones
+    // tiles of an operator: 256 / fmt rows for CSR operators, runs of whole slices for SELL ones
     struct Launch {
         Tiles first;
         int second; // grid

@@ -52,7 +52,8 @@ struct Tuning {
                                 // the current row is summed (0: one row at a time)
     int col16 = 0;              // FP32 operators store 16-bit column offsets where they fit
     int tail_rows = 0;          // coarse levels of at most this many rows (and everything below
-                                // them) run as one persistent tail kernel; 0 disables it
+                                // them) run as one persistent tail kernel, as far up as their
+                                // operators are CSR lane groups; 0 disables it
     int pdl = 1;                // programmatic dependent launch between consecutive kernels
     int wait_polls = 1 << 22;   // poll limit of the bounded device waits (< 0: give up at once)
     int mixed_sweeps = 0;       // mixed precision: Jacobi sweeps per level (0: the hierarchy's)
@@ -233,7 +234,10 @@ private:
     int vcycle_visit(const DevSell64_32& m) const {
         const bool fp64 = m.s64.val != nullptr;
         const int fmt = fp64 ? m.s64.fmt : m.s32.fmt;
-        if (fmt == kFmtSell && tuning_.vcycle_pair) return krylov_visit_of(row_width(m), true);
+        const bool ahead = fmt == kFmtSell && tuning_.vcycle_pair != 0;
+        // these step by kBlock (Visit)
+        if ((ahead || fmt != kFmtSell) && m.threads != kBlock) fail(7, "engine: a strategy of 256 threads on smaller CTAs");
+        if (ahead) return krylov_visit_of(row_width(m), true);
         return visit_of(fmt, row_width(m), static_cast<int>(static_cast<long long>(m.n_tiles) * m.threads / kBlock), fp64 && !need32_);
     }
     // stored entries per row of a SELL operator

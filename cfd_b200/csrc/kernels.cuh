@@ -10,8 +10,10 @@
 //
 // Work decomposition: each level's rows are concatenated over the systems of a batch (a single
 // solve is a batch of one), each system's block padded to a multiple of 32 rows. A tile is a
-// run of whole slices of ONE system; one CTA of 256 threads processes one tile. Tiles carry
-// their system id so converged systems are skipped and reductions stay per system.
+// run of rows of ONE system, processed by one CTA: of 256 threads (kBlock), or of 128 for the
+// V-cycle kernels of FP64 SELL operators of long rows (Engine::build, op_tiles). What needs
+// kBlock threads says so. Tiles carry their system id so converged systems are skipped and
+// reductions stay per system.
 //
 // Reductions (CG dot products) are deterministic: each tile writes its partial sums, the last
 // CTA of a system to finish (atomic ticket) adds that system's partials in a fixed order and
@@ -25,8 +27,10 @@
 namespace cfdb {
 
 constexpr int kBlock = 256;
-// Rows of a SELL tile of the V-cycle kernels (one row per thread); also the window within which
-// a SELL operator's rows may be reordered by length.
+// Unit of the SELL tiles: level-0 Krylov tiles are multiples of it, V-cycle tiles multiples of it or of
+// its half (CTAs of 128 threads). Also the window within which a SELL operator's rows may be
+// reordered by length: positions of a window stay in it, so any tile of whole slices visits
+// each of its rows once.
 constexpr int kSellRows = kBlock;
 
 // Programmatic dependent launch (sm_90+): pdl_launch lets the next kernel of the stream be
@@ -50,9 +54,9 @@ __device__ __forceinline__ void pdl_entry() {
 //     order.
 //  G in {4, 8, 16, 32, 64, 128, 256}: CSR with G lanes per row; `slice` = row offsets. Used
 //     for wide coarse-level rows (tens to thousands of entries) and for operators of few rows,
-//     where one thread per row would serialise long load chains; lanes sum strided entries and combine them with a fixed
-//     butterfly (and, above 32 lanes, a fixed-order sum over the row's warps): deterministic,
-//     but not the sequential CSR order. Tiles of a CSR operator hold 256 / G rows (8-row tiles
+//     where one thread per row would serialise long load chains; lanes sum strided entries and
+//     combine them with a fixed butterfly (and, above 32 lanes, a fixed-order sum over the row's
+//     warps): deterministic, but not the sequential CSR order. Tiles of a CSR operator hold 256 / G rows (8-row tiles
 //     of 8 G threads took 28 us instead of 8.5 us on 217K rows of 17 entries with G = 4: CTAs of
 //     one warp fill half of an SM's warp slots).
 enum : int { kFmtSell = 0 };
@@ -128,7 +132,7 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Block-wide sum of two values; result valid in thread 0. Fixed tree: deterministic.
+// Block-wide sum of two values over kBlock threads; result valid in thread 0. Fixed tree: deterministic.
 __device__ __forceinline__ void block_sum2(double& a, double& b) {
     __shared__ double sa[kBlock / 32], sb[kBlock / 32];
     a = warp_sum(a);
@@ -453,8 +457,9 @@ __device__ __forceinline__ T csr_lane_sum(const Sell<T>& m, int G, CsrQuads<T>& 
 }
 
 // CSR row sum by a group of G lanes (G a power of two dividing 32), each with its first pass over
-// the row loaded (csr_begin); partial sums are combined with a fixed butterfly over the group. Every lane of the group returns the same total. All
-// lanes of the warp must call it (the shuffles use the full mask).
+// the row loaded (csr_begin); partial sums are combined with a fixed butterfly over the group.
+// Every lane of the group returns the same total. All lanes of the warp must call it (the shuffles
+// use the full mask).
 template <class T, class XA>
 __device__ __forceinline__ T csr_group_sum(const Sell<T>& m, CsrQuads<T>& q, bool valid, int G, XA xa) {
     T s = valid ? csr_lane_sum(m, G, q, xa) : T(0);
@@ -511,7 +516,9 @@ constexpr int kBatch = V == kVisitSell4 ? 4 : V == kVisitSell5 || V == kVisitStr
 
 // One tile's visit: begin() issues the loads of the thread's first row that depend on the
 // operator alone (before pdl_wait); run() calls f(row, sum_j a_row,j xa(j), e) for every row of
-// the tile, with the row's other operands e = pre(row) loaded ahead of its gathers.
+// the tile, with the row's other operands e = pre(row) loaded ahead of its gathers. The stream and
+// the CSR strategies step by kBlock and need blocks of that many threads; the other SELL strategies
+// step by blockDim.x.
 //
 // What bounds these kernels is the chain of dependent loads of a row (slice offsets, columns and
 // values, gathers) against the few rows that a thread has in flight, so a row's entries are taken

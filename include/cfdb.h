@@ -160,8 +160,9 @@ typedef struct cfdb_hierarchy cfdb_hierarchy;
 int cfdb_amg_setup(const cfdb_csr* a, const cfdb_amg_settings* settings,
                    cfdb_hierarchy** out);
 /* The same hierarchy built on the device (sparse products, strength graph, transfers and
- * Galerkin operators in CUDA kernels; the aggregation too, except on small or dense levels and
- * where many rows are left for its third pass), bit-identical to cfdb_amg_setup. */
+ * Galerkin operators in CUDA kernels; the aggregation too, except on small or dense levels, with
+ * columns that very many rows are strongly connected to, where many rows are left for its third
+ * pass, and where device memory is short), bit-identical to cfdb_amg_setup. */
 int cfdb_amg_setup_device(const cfdb_csr* a, const cfdb_amg_settings* settings,
                           cfdb_hierarchy** out);
 int cfdb_hierarchy_destroy(cfdb_hierarchy* h);
@@ -372,11 +373,13 @@ int cfdb_system_assemble_device(cfdb_system* sys, const double* flux, const doub
                                 double* lower, double* diag, double* divergence);
 /* AmgPreconditioner::apply (amg.hpp:33; accelerator V-cycle krylov_kernels.inc:209-238): one
  * V-cycle z = M^-1 r with zero initial guess on the installed hierarchy and the current
- * matrix (set by the last solve), in the system's precision. Host arrays. */
+ * matrix (set by the last solve, also by one that returned at once), in the system's precision.
+ * Host arrays. */
 int cfdb_system_apply_amg(cfdb_system* sys, const double* r, double* z);
 /* Ordered arithmetic: every level operator stored for thread-per-row sums in the CSR column
  * order, so FP64 V-cycles are bit-identical to the reference's sequential host arithmetic
- * (slower on wide coarse levels). Default off: wide coarse rows use warp-per-row sums. */
+ * (slower on coarse levels). Default off: long rows, and those of small operators, are summed by
+ * groups of lanes. */
 int cfdb_system_set_ordered(cfdb_system* sys, int ordered);
 
 /* Per-kernel device time of the initial residual plus one iteration (events around
@@ -436,7 +439,8 @@ typedef struct {
     int krylov_pair;  /* level-0 Krylov SpMV kernels load a thread's next row while they sum the current
                          one (1, default), or take one row at a time (0) */
     int tail_rows;    /* coarse levels of at most this many rows, with all coarser ones, run as one
-                         persistent kernel; 0 (default) disables it */
+                         persistent kernel as far up as all their operators are CSR lane groups;
+                         0 (default) disables it */
     int col16;        /* FP32 operators keep 16-bit column offsets from a per-slice / per-row base
                          where every slice / row spans fewer than 65536 columns, default 0 */
     int pdl;          /* programmatic dependent launch between consecutive kernels (a kernel is
