@@ -1454,12 +1454,15 @@ DevCsr prune_zeros(Ctx& cx, const DevCsr& a) {
 // Rows left by pass 2 that pass 3 runs on the device (one thread); more go to the host.
 constexpr int kPass3Device = 1024;
 
-// Levels aggregated on the device: all but the small and the dense ones (the conflict lists grow with
-// the square of the strong entries per row, while the host's sequential pass costs nanoseconds per
-// strong entry plus the strength graph's read-back). Measured, aggregation phase of all levels with
-// the host from 262K rows or 6 strong entries per row down, against this line: tet 95^3x6 22.1 / 14.9
-// ms (its second level: 861K rows of 8.7), tet 50^3x6 4.4 / 3.6, tet 30^3x6 1.9 / 1.3, graded 64^3 2.6 / 2.1.
-bool device_aggregation(int n, long long ns) { return n >= 4096 && ns <= 20LL * n; }
+// Levels aggregated on the device: those of at least 200K strong entries, but not the dense ones (the
+// conflict lists grow with the square of the strong entries per row). The device's time is that of a chain of
+// decisions and of some 20 launches, 0.3 to 0.6 ms on the smallest levels; the host's is a few nanoseconds a
+// strong entry plus the strength graph's read-back. Measured, one level, device / host in us (strong
+// entries, per row): 23K, 5.6: 358 / 116; 94K, 3.8: 345 / 252; 91K, 9.8: 661 / 384; 156K, 9.8: 742 / 624; 190K,
+// 5.8: 574 / 235 (box) and 576 / 269 (graded); 237K, 8.6: 782 / 978; 326K, 9.6: 1109 / 1289; 350K, 11.0:
+// 1313 / 1261; 374K, 5.8: 725 / 742 (box) and 710 / 954 (graded); 632K, 3.9: 520 / 841; 1.9M, 8.7:
+// 1811 / 3178; 2.9M, 3.9: 1113 / 3620.
+bool device_aggregation(int n, long long ns) { return ns >= 200000 && ns <= 20LL * n; }
 
 // The aggregation on the device from the strength graph (srp, sci, sav = |a_ij|): passes 1 and
 // 2 in parallel, pass 3 by one thread when at most kPass3Device rows are left for it. agg

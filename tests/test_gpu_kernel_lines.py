@@ -168,12 +168,12 @@ def _abs_matvec(a, x):
     return np.add.reduceat(np.abs(a.va) * np.abs(x)[a.ci], a.rp[:-1])
 
 
-@pytest.mark.parametrize("n", [4095, 4097, 9000])
+@pytest.mark.parametrize("n", [4095, 4097, 9000, 70000])
 @pytest.mark.parametrize("half", [3, 4, 7, 8, 9, 10, 15, 16])
 def test_setup_at_the_row_lengths_of_its_kernels(gpu, n, half):
     """Rows of 2 half + 1 entries: products of 7 to 33 contributions (8, 16 and 32 lanes, then
-    tables), sorts of up to 32 entries and more, aggregation of levels around 4096 rows and 20
-    strong entries a row. Every level equals the host build bit for bit."""
+    tables), sorts of up to 32 entries and more, aggregation on the device (70000 rows, up to 20 strong
+    entries a row) and on the host. Every level equals the host build bit for bit."""
     cb = gpu
     own, nei, up, lo, diag, _ = _banded(n, half, seed=half)
     a = _csr(n, own, nei, diag, up, lo)
@@ -283,14 +283,15 @@ def _same_hierarchies(d, h):
     assert np.array_equal(d.coarse_inverse(), h.coarse_inverse())
 
 
-@pytest.mark.parametrize("n", [4095, 4096, 9000])
-@pytest.mark.parametrize("per_row", [1, 2, 4, 6, 12])
+@pytest.mark.parametrize("n,per_row", [(66000, 1), (70000, 1), (33000, 2), (36000, 2), (16000, 4), (20000, 4),
+                                       (11000, 6), (14000, 6), (9000, 12)])
 def test_setup_with_repeated_columns(gpu, n, per_row):
-    """A CSR matrix whose rows (of about 4 to 40 entries) hold some columns twice: the device setup
-    treats them as separate entries, as the host build does, and equals it bit for bit, every time."""
+    """A CSR matrix whose rows (of about 4 to 40 entries) hold some columns twice, of 190K to 250K strong
+    entries and so on either side of the device aggregation's line: the device setup treats the copies as
+    separate entries, as the host build does, and equals it bit for bit, every time."""
     cb = gpu
     view = cb.CsrView(n, *_scattered(n, per_row, seed=per_row))
-    s = cb.AmgSettings(strength_threshold=0.0, max_levels=3)
+    s = cb.AmgSettings(strength_threshold=0.0)
     h = cb.AmgHierarchy(view, s)
     for _ in range(2):
         _same_hierarchies(cb.AmgHierarchy(view, s, device=True), h)
@@ -371,16 +372,16 @@ def _with_hub(n, half, degree, seed=9):
     return _csr(n, own[o], nei[o], diag, v, v.copy())
 
 
-@pytest.mark.parametrize("n,degree", [(9000, 300), (9000, 1200), (9000, 1400), (9000, 8900), (60000, 59000)])
+@pytest.mark.parametrize("n,degree", [(40000, 300), (40000, 2800), (40000, 3600), (40000, 39000), (150000, 149000)])
 def test_setup_with_a_hub_row(gpu, n, degree):
     """One row strongly connected to many: its rows conflict pairwise (degree^2 / 2), which the device
-    aggregates up to 24 conflicts a strong entry (degrees to about 1300 of 9000 rows) and the host beyond.
+    aggregates up to 24 conflicts a strong entry (degrees to about 3200 of 40000 rows) and the host beyond.
     Equal to the host build, within memory in proportion to the matrix."""
     import torch
     cb = gpu
-    a = _with_hub(n, 2, degree)
+    a = _with_hub(n, 3, degree)
     view = cb.CsrView(a.n_rows, a.rp, a.ci, a.va)
-    s = cb.AmgSettings(strength_threshold=0.0, max_levels=2)
+    s = cb.AmgSettings(strength_threshold=0.0)
     h = cb.AmgHierarchy(view, s)
     free = torch.cuda.mem_get_info()[0]
     _same_hierarchies(cb.AmgHierarchy(view, s, device=True), h)
