@@ -21,6 +21,8 @@
 // pass; a bitonic sort of the table then yields the row's columns in ascending order.
 #include "dsetup.hpp"
 
+#include "aggregation_rule.hpp"
+
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -292,6 +294,8 @@ __global__ void k_max_degree(int n, const int* __restrict__ srp, int* out) {
 // so that a link costs about one L2 load. Walking the graph and its transpose for every look cost 20
 // to 30 dependent loads a link: 288 sweeps of one look, 3.7 ms, on the 750K-cell tet box. The looks are
 // bounded and nothing depends on how far they get: a row still waiting is left to the next sweep.
+// A long thin mesh, or a matrix close to a band, makes chains of thousands of links, of which a sweep
+// passes some 25: slow_sweeps hands such a level to the host.
 enum : int { kUndecided = 0, kSeed = 1, kNotSeed = 2 };
 
 __global__ void k_seed_init(int n, const int* __restrict__ srp, int* state) {
@@ -365,11 +369,11 @@ __global__ void k_conflicts(int n, const int* __restrict__ srp, const int* __res
 
 // One sweep over the rows [lo, lo + kSeedWindow), lo = *lo_in (every row below it is decided);
 // *lo_out receives the smallest row still undecided, or lo + kSeedWindow when the window
-// settled (*lo_out preset to INT_MAX). crp / cci: the earlier conflicts; at[i]: how many of row i's
+// settled (*lo_out preset to INT_MAX); *done += the rows decided here. crp / cci: the earlier conflicts; at[i]: how many of row i's
 // are known not to be seeds (kept between sweeps). The loop is flat, one look per turn, so that the
 // lanes of a warp that can decide are never held back by waiting ones.
 __global__ void k_seed_sweep(int n, const int* __restrict__ lo_in, int* lo_out, const int* __restrict__ crp,
-                             const int* __restrict__ cci, int* at, int* state_) {
+                             const int* __restrict__ cci, int* at, int* state_, int* done) {
     const int lo = *lo_in;
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicMin(lo_out, static_cast<int>(min(static_cast<long long>(lo) + kSeedWindow, static_cast<long long>(n))));
@@ -377,6 +381,7 @@ __global__ void k_seed_sweep(int n, const int* __restrict__ lo_in, int* lo_out, 
     volatile int* state = state_;
     const int i = ii < n ? static_cast<int>(ii) : 0;
     bool open = ii < n && state[i] == kUndecided;
+    const bool was_open = open;
     int pos = 0, end = 0;
     bool blocked = false; // c[0] was undecided at the last look
     int c[kSeedLook];
@@ -414,6 +419,8 @@ __global__ void k_seed_sweep(int n, const int* __restrict__ lo_in, int* lo_out, 
     if (open) at[i] = pos - crp[i];
     const int left = __reduce_min_sync(0xffffffffu, open ? i : INT_MAX);
     if (left != INT_MAX && (threadIdx.x & 31) == 0) atomicMin(lo_out, left);
+    const int decided = __syncthreads_count(was_open && !open);
+    if (threadIdx.x == 0 && decided > 0) atomicAdd(done, decided);
 }
 
 __global__ void k_seed_flags(int n, const int* __restrict__ state, int* flag) {
@@ -1454,22 +1461,12 @@ DevCsr prune_zeros(Ctx& cx, const DevCsr& a) {
 // Rows left by pass 2 that pass 3 runs on the device (one thread); more go to the host.
 constexpr int kPass3Device = 1024;
 
-// Levels aggregated on the device: those of at least 200K strong entries, but not the dense ones (the
-// conflict lists grow with the square of the strong entries per row). The device's time is that of a chain of
-// decisions and of some 20 launches, 0.3 to 0.6 ms on the smallest levels; the host's is a few nanoseconds a
-// strong entry plus the strength graph's read-back. Measured, one level, device / host in us (strong
-// entries, per row): 23K, 5.6: 358 / 116; 94K, 3.8: 345 / 252; 91K, 9.8: 661 / 384; 156K, 9.8: 742 / 624; 190K,
-// 5.8: 574 / 235 (box) and 576 / 269 (graded); 237K, 8.6: 782 / 978; 326K, 9.6: 1109 / 1289; 350K, 11.0:
-// 1313 / 1261; 374K, 5.8: 725 / 742 (box) and 710 / 954 (graded); 632K, 3.9: 520 / 841; 1.9M, 8.7:
-// 1811 / 3178; 2.9M, 3.9: 1113 / 3620.
-bool device_aggregation(int n, long long ns) { return ns >= 200000 && ns <= 20LL * n; }
-
 // The aggregation on the device from the strength graph (srp, sci, sav = |a_ij|): passes 1 and
 // 2 in parallel, pass 3 by one thread when at most kPass3Device rows are left for it. agg
 // receives every row's aggregate. Returns the number of aggregates, or -1 when more rows are
 // left for pass 3 (isolated rows, or rows none of whose strong neighbours pass 1 aggregated), when the
-// conflict lists pass kConflictsPerStrong or 2^31 entries, or when there is no memory for them: the
-// caller then aggregates on the host.
+// conflict lists pass kConflictsPerStrong or 2^31 entries, when its rows decide too much one after
+// another (slow_sweeps), or when there is no memory for the lists: the caller then aggregates on the host.
 int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, int* agg) {
     cudaStream_t st = cx.st;
     // scratch of its own (the transpose, conflict lists), given back before the products need theirs and
@@ -1505,22 +1502,25 @@ int aggregate_device(Ctx& cx, int n, int ns, int* srp, int* sci, double* sav, in
     k_conflicts<true><<<grid_for(n), kThreads, 0, st>>>(n, srp, sci, t.rp, t.ci, nullptr, crp, cci, nullptr, 0);
     int* at = ccnt; // conflicts passed so far
     CFDB_CUDA(cudaMemsetAsync(at, 0, sizeof(int) * static_cast<size_t>(n), st));
-    // lo of each sweep of a batch; lo[0] = 0, then the last lo of the previous batch
-    int* lo = tx.mem->alloc<int>(kSeedBatch + 1);
-    CFDB_CUDA(cudaMemsetAsync(lo, 0, sizeof(int), st));
+    // lo of each sweep of a batch (lo[0] = 0, then the last lo of the previous batch), and behind them
+    // the rows decided in all sweeps
+    int* lo = tx.mem->alloc<int>(kSeedBatch + 2);
+    int* done = lo + kSeedBatch + 1;
+    CFDB_CUDA(cudaMemsetAsync(lo, 0, sizeof(int) * (kSeedBatch + 2), st));
     const int grid = grid_for(std::min(n, kSeedWindow));
     for (long long sweeps = 0;;) {
         // in every sweep its smallest undecided row is decided, or passes kSeedPolls x kSeedLook of its conflicts
         if (sweeps > n + n_conf / (kSeedPolls * kSeedLook) + kSeedBatch) fail(kErrInternal, "device aggregation did not settle");
         CFDB_CUDA(cudaMemsetAsync(lo + 1, 0x7f, sizeof(int) * kSeedBatch, st));
         for (int b = 0; b < kSeedBatch; ++b)
-            k_seed_sweep<<<grid, kThreads, 0, st>>>(n, lo + b, lo + b + 1, crp, cci, at, state);
+            k_seed_sweep<<<grid, kThreads, 0, st>>>(n, lo + b, lo + b + 1, crp, cci, at, state, done);
         CFDB_CUDA(cudaGetLastError());
         sweeps += kSeedBatch;
-        int last = 0;
-        CFDB_CUDA(cudaMemcpyAsync(&last, lo + kSeedBatch, sizeof(int), cudaMemcpyDeviceToHost, st));
+        int last[2] = {0, 0}; // the last lo, and *done
+        CFDB_CUDA(cudaMemcpyAsync(last, lo + kSeedBatch, sizeof(last), cudaMemcpyDeviceToHost, st));
         sync(st);
-        if (last >= n) break;
+        if (last[0] >= n) break;
+        if (slow_sweeps(sweeps, n, ns, std::max(last[0], last[1]))) return -1;
         CFDB_CUDA(cudaMemcpyAsync(lo, lo + kSeedBatch, sizeof(int), cudaMemcpyDeviceToDevice, st));
     }
     int* flag = tx.mem->alloc<int>(static_cast<size_t>(n) + 1);

@@ -161,8 +161,9 @@ int cfdb_amg_setup(const cfdb_csr* a, const cfdb_amg_settings* settings,
                    cfdb_hierarchy** out);
 /* The same hierarchy built on the device (sparse products, strength graph, transfers and
  * Galerkin operators in CUDA kernels; the aggregation too, except on small or dense levels, with
- * columns that very many rows are strongly connected to, where many rows are left for its third
- * pass, and where device memory is short), bit-identical to cfdb_amg_setup. */
+ * columns that very many rows are strongly connected to, where its rows decide one after another
+ * (long thin meshes), where many rows are left for its third pass, and where device memory is
+ * short), bit-identical to cfdb_amg_setup. */
 int cfdb_amg_setup_device(const cfdb_csr* a, const cfdb_amg_settings* settings,
                           cfdb_hierarchy** out);
 int cfdb_hierarchy_destroy(cfdb_hierarchy* h);

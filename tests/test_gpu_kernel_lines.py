@@ -476,3 +476,19 @@ def test_mixed_batch_with_a_target_out_of_reach(gpu):
     for i in (0, 2):
         assert out[1e-8][1][i] == out[1e-18][1][i]
         assert np.array_equal(out[1e-8][0][i * n:(i + 1) * n], out[1e-18][0][i * n:(i + 1) * n])
+
+
+@pytest.mark.parametrize("shape", [(150000, 1, 1), (3, 3, 9000), (9000, 3, 3), (300, 300, 1), (40, 40, 40)])
+def test_setup_of_long_thin_meshes(gpu, shape):
+    """Meshes whose rows decide one after another along their length, for which the device leaves the
+    aggregation to the host after some sweeps, and two that settle on the device: equal to the host build."""
+    cb = gpu
+    m = cb.Mesh.box(*shape)
+    ni, n = m.n_internal_faces, m.n_cells
+    own, nei = np.ascontiguousarray(m.owner[:ni]), m.neighbour
+    w = np.random.default_rng(1).uniform(0.5, 1.5, ni)
+    diag = np.bincount(own, w, n) + np.bincount(nei, w, n) + 0.01
+    a = _csr(n, own, nei, diag, -w, -w.copy())
+    view = cb.CsrView(a.n_rows, a.rp, a.ci, a.va)
+    s = cb.AmgSettings(strength_threshold=0.04)
+    _same_hierarchies(cb.AmgHierarchy(view, s, device=True), cb.AmgHierarchy(view, s))
